@@ -21,6 +21,7 @@
 #include "aux_kernels.cuh"
 #include "hippolbm.h"
 #include "launch.cuh"
+#include "lbm_step_resident.cuh"
 
 using namespace hlbm;
 
@@ -126,6 +127,8 @@ struct hlbm_ctx {
   int8_t* nearwall = nullptr;  // per node: some pull comes from a wall node (k_near_wall)
   bool maybe_walls = false;     // the flags may hold wall nodes (an obstacle was rasterised or put)
   bool variant_tuned = false;   // hlbm_tune / hlbm_autotune chose the variant (else the tier default)
+  bool variant_forced = false;  // hlbm_tune chose it: the step kernel of that variant runs, never the resident one
+  unsigned* group_dev = nullptr;  // many-step launches: CTAs that have left, and 128 bytes on the barrier counter
   long long wait_limit = TMA_WAIT_LIMIT;  // polls before a wait of the pipelined kernel gives up
   double* partials = nullptr;
   double* stats_dev = nullptr;
@@ -258,8 +261,10 @@ int setup_pipeline(hlbm_ctx* c) {
   const StepPlan& p = c->plan;
   if (!c->plan_dev) {
     if (pool_alloc((void**)&c->plan_dev, sizeof(StepPlan), c->device, c->stream) != cudaSuccess ||
-        pool_alloc((void**)&c->desc_dev, sizeof(LatticeDesc), c->device, c->stream) != cudaSuccess)
+        pool_alloc((void**)&c->desc_dev, sizeof(LatticeDesc), c->device, c->stream) != cudaSuccess ||
+        pool_alloc((void**)&c->group_dev, 256, c->device, c->stream) != cudaSuccess)
       return fail(HLBM_ENOMEM, "cannot allocate the step plan");
+    HLBM_CK(cudaMemsetAsync(c->group_dev, 0, 256, c->stream));
   }
   HLBM_CK(cudaMemcpyAsync(c->plan_dev, &p, sizeof(StepPlan), cudaMemcpyHostToDevice, c->stream));
   LatticeDesc d{};
@@ -334,16 +339,28 @@ int build_plan(hlbm_ctx* c) {
       }
     }
   }
+  int recorded = 0;
   for (int stage : {HLBM_HOOK_POST_STREAM, HLBM_HOOK_BOUNDARY_CONDITIONS}) {
     for (const HookOp& h : c->hooks) {
       if (h.hook != stage) continue;
-      if (p.nops >= MAX_PLANE_OPS) return fail(HLBM_EPLAN, "too many boundary operators");
+      if (recorded++ >= MAX_PLANE_OPS) return fail(HLBM_EPLAN, "too many boundary operators");
       PlaneOp& op = p.ops[p.nops];
       if (h.kind == H_POST_BB) {
         if (!pre_seen)
           return fail(HLBM_EPLAN,
                       "post_bounce_back needs pre_bounce_back in pre_stream_bcs (it restores the saved populations)");
-        op.kind = OP_POST_BB;
+        // While no neumann / lid has changed the pulled values they are the ones this operator
+        // restores (on-node bounce-back; the zero-gradient passes write what the pull reads), so only
+        // the z faces' increments are left, and a second post_bounce_back changes nothing.  Without
+        // increments FP64 and FP32 need no operator on the faces of a closed box (the 16-bit tiers:
+        // face_pass_mask), and the node code no longer reloads the five slots of each face.
+        bool restored = false, leading = true;
+        for (int o = 0; o < p.nops; o++) {
+          restored |= p.ops[o].kind == OP_CAVITY;
+          leading &= p.ops[o].kind == OP_CAVITY || p.ops[o].kind == OP_ZERO_GRADIENT;
+        }
+        if (leading && (restored || (p.ncav[4] + p.ncav[5] == 0 && elem_size(c->precision) > 2))) continue;
+        op.kind = leading ? OP_CAVITY : OP_POST_BB;
         op.face = 0;
       } else if (h.kind == H_ZERO_GRADIENT) {
         op.kind = OP_ZERO_GRADIENT;
@@ -368,7 +385,7 @@ int build_plan(hlbm_ctx* c) {
     }
     b.value = h.value;
   }
-  p.face_mask = face_pass_mask(p);
+  p.face_mask = face_pass_mask(p, int(elem_size(c->precision)));
   if (int rc = setup_pipeline(c)) return rc;
   c->plan_dirty = false;
   c->plan_version++;
@@ -384,6 +401,57 @@ cudaError_t outlet_passes(int prec, const StepPlan& p, const LatticeDesc* descs,
     if (cudaError_t e = launch_zero_gradient(prec, descs, m, p.ops[o].face, parity, n, s)) return e;
   }
   return cudaSuccess;
+}
+
+// Whether a lattice steps in the resident kernel (lbm_step_resident.cuh): both population buffers
+// together within this many bytes, a plan it takes, and no variant asked for by hlbm_tune.  Measured
+// (us a step, resident against one launch a step): FP64 24^3 3.0 / 6.3, 64^3 (80 MB) 14.1 / 14.5, 80^3
+// (156 MB) 40 / 30; FP32 24^3 2.6 / 11.4, 80^3 (78 MB) 17.2 / 24.9, 96^3 (134 MB) 42 / 39; FP16 24^3
+// 3.1 / 20.6, 80^3 (39 MB) 18.5 / 23.7, 96^3 (67 MB) 29.8 / 26.7 (the row pipeline copies in bulk).
+// 16-bit MRT keeps its step kernels: there the node-pair form of every kernel has to round alike.
+constexpr int64_t resident_bytes(int precision) {
+  return int64_t(precision == HLBM_F16 || precision == HLBM_BF16 ? 50 : 100) << 20;
+}
+bool resident_applies(const hlbm_ctx* c) {
+  const bool half = elem_size(c->precision) == 2;
+  return !c->variant_forced && resident_plan(c->plan) && !(half && c->collision == 1) &&
+         2 * int64_t(Q) * c->ncell * int64_t(elem_size(c->precision)) <= resident_bytes(c->precision);
+}
+
+cudaError_t launch_resident_tier(int precision, const ResidentArgs& a, int walls, cudaStream_t s) {
+  switch (precision) {
+    case HLBM_F64: return resident_f64(a, walls, s);
+    case HLBM_F64_STRICT: return resident_f64_strict(a, walls, s);
+    case HLBM_F32: return resident_f32(a, walls, s);
+    case HLBM_F16: return resident_f16(a, walls, s);
+    default: return resident_bf16(a, walls, s);
+  }
+}
+
+// nsteps fused steps of one lattice in resident launches of at most RESIDENT_STEPS (a step of the
+// largest lattice taken is some 40 us, and the waits of a launch give up after two seconds)
+constexpr int RESIDENT_STEPS = 1024;
+int resident_steps(hlbm_ctx* c, int64_t nsteps) {
+  ResidentArgs a;
+  a.descs = c->desc_dev;
+  a.left = c->group_dev;
+  a.bars = c->group_dev + RES_BAR_STRIDE;
+  a.nbars = 1;
+  a.err = c->err_dev;
+  a.grid = int(std::min<int64_t>(c->sms, (c->ncell + 63) / 64));
+  a.wait_limit = c->wait_limit;
+  while (nsteps > 0) {
+    const int m = int(std::min<int64_t>(nsteps, RESIDENT_STEPS));
+    a.one = ResidentTask{0, 0, a.grid, 0, m};
+    a.parity = c->cur;  // the descriptor holds f[0], f[1] with cur = 0
+    a.seed = uint32_t(c->steps);
+    c->launches++;
+    HLBM_CK(launch_resident_tier(c->precision, a, c->plan.walls, c->stream));
+    if (m & 1) c->cur = 1 - c->cur;
+    c->steps += m;
+    nsteps -= m;
+  }
+  return HLBM_OK;
 }
 
 // One step (or read-out) of lattice c with plan p on stream s: the outlet passes, then the step
@@ -564,10 +632,10 @@ int hlbm_domain(const int32_t cell_dims[3], const double bmin[3], const double b
     cudaGetLastError();
     return cleanup(fail(HLBM_ENOMEM, "hlbm_domain: cannot allocate the error word"));
   }
-  // the flag bytes are padded to 128 (the span pipeline bulk-copies whole 16-byte chunks of them)
+  // flag and map bytes are padded to 128 (the pipelines bulk-copy whole 16-byte chunks of the map)
   const size_t flag_bytes = size_t((c->ncell + 127) / 128 * 128);
   if (pool_alloc((void**)&c->flags, flag_bytes, c->device, c->stream) != cudaSuccess ||
-      pool_alloc((void**)&c->nearwall, size_t(c->ncell), c->device, c->stream) != cudaSuccess ||
+      pool_alloc((void**)&c->nearwall, flag_bytes, c->device, c->stream) != cudaSuccess ||
       pool_alloc((void**)&c->partials, sizeof(double) * 4 * 148 * 8, c->device, c->stream) != cudaSuccess ||
       pool_alloc((void**)&c->stats_dev, sizeof(double) * 4, c->device, c->stream) != cudaSuccess) {
     cudaGetLastError();
@@ -575,7 +643,7 @@ int hlbm_domain(const int32_t cell_dims[3], const double bmin[3], const double b
   }
   // init_obst: every flag FLUIDE_ (-1 = 0xff)
   if (cudaMemsetAsync(c->flags, 0xff, flag_bytes, c->stream) != cudaSuccess ||
-      cudaMemsetAsync(c->nearwall, 0, size_t(c->ncell), c->stream) != cudaSuccess)
+      cudaMemsetAsync(c->nearwall, 0, flag_bytes, c->stream) != cudaSuccess)
     return cleanup(fail(HLBM_ECUDA, "cudaMemsetAsync failed"));
   // default lbm_parameters slots (lbm_parameters.cpp:57-64)
   const double F0[3] = {0, 0, 0};
@@ -592,7 +660,7 @@ int hlbm_destroy(hlbm_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) {  // the memory returns to the pool once the stream's work is done
     void* bufs[] = {c->f[0], c->f[1], c->flags, c->nearwall, c->partials, c->stats_dev, c->plane_tmp, c->uprev,
-                    c->plan_dev, c->desc_dev, c->tiles_dev, c->err_dev, c->seed_dev};
+                    c->plan_dev, c->desc_dev, c->tiles_dev, c->err_dev, c->seed_dev, c->group_dev};
     for (void* b : bufs) pool_free(b, c->stream);
     cudaStreamDestroy(c->stream);
   }
@@ -886,6 +954,7 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
     c->steps++;
     nsteps--;
   }
+  if (nsteps > 0 && resident_applies(c)) return resident_steps(c, nsteps);
   for (int64_t s = 0; s < nsteps; s++) {
     HLBM_CK(launch_step_kernel(c, MODE_FUSED, c->f[c->cur], c->f[1 - c->cur]));
     c->cur = 1 - c->cur;
@@ -1197,7 +1266,7 @@ int hlbm_tune(hlbm_ctx* c, int32_t variant) {
   if (!c || variant < 0 || variant >= NUM_VARIANTS)
     return fail(HLBM_EINVAL, "hlbm_tune: variant must be in [0, " + std::to_string(NUM_VARIANTS) + ")");
   c->variant = variant;
-  c->variant_tuned = true;
+  c->variant_tuned = c->variant_forced = true;
   return HLBM_OK;
 }
 
@@ -1218,7 +1287,7 @@ int hlbm_autotune(hlbm_ctx* c, int32_t reps, int32_t* chosen, double* ms_per_var
     if (ms_per_variant) ms_per_variant[v] = -1.0;
     if (v < 6 && (v % 2) == 1 && !vec_applies(c, v)) continue;
     if (v >= 8 && !rows_runs(c->plan, v, MODE_FUSED, int(elem_size(c->precision)))) continue;
-    if (v >= 6 && c->tma_stages < 2) continue;
+    if ((v == 6 || v == 7) && c->tma_stages < 2) continue;
     cudaError_t e = launch_step_variant(c, MODE_FUSED, fin, fout, v);  // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
     for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch_step_variant(c, MODE_FUSED, fin, fout, v);

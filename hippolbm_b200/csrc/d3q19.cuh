@@ -29,13 +29,19 @@ struct PlaneBB {
 };
 
 // Step plan: the node-local form of the operator lists of one deck.
-enum OpKind : int32_t { OP_POST_BB = 0, OP_ZOUHE = 1, OP_LID = 2, OP_SETDIST = 3, OP_ZERO_GRADIENT = 4 };
+// OP_CAVITY: the part of a leading post_bounce_back that the pull has not done already.  On a
+// non-periodic face the pull bounces on the node, i.e. it reads the very values post_bounce_back
+// restores, so while no other operator has changed the node's values only the cavity increments of
+// the z faces are left (capi.cu: build_plan).
+enum OpKind : int32_t {
+  OP_POST_BB = 0, OP_ZOUHE = 1, OP_LID = 2, OP_SETDIST = 3, OP_ZERO_GRADIENT = 4, OP_CAVITY = 5
+};
 constexpr int MAX_PLANE_OPS = 16;
 constexpr int MAX_CAVITY = 4;
 constexpr int MAX_SETS = 8;
 
 struct PlaneOp {
-  int32_t kind;  // OP_POST_BB (all non-periodic faces), OP_ZOUHE / OP_LID (one face)
+  int32_t kind;  // OP_POST_BB (all non-periodic faces), OP_CAVITY (z faces), OP_ZOUHE / OP_LID (one face)
   int32_t face;  // 0..5
   double u[3];   // lattice units
 };
@@ -127,15 +133,21 @@ inline bool face_pass_runs(const StepPlan& p, int walls, int variant, bool prolo
 }
 
 // Faces whose nodes the boundary operators of the plan can change: every non-periodic face for
-// post_bounce_back, the operator's own face for neumann / lid_driven_cavity.  Bit F = face F
+// post_bounce_back after another operator, the z faces with increments for a leading one, the
+// operator's own face for neumann / lid_driven_cavity.  The 16-bit tiers (bytes 2) keep every
+// non-periodic face for a leading one too: their operators work on full populations, and converting
+// there and back rounds, so leaving nodes out would change the stored state.  Bit F = face F
 // (x0, xl, y0, yl, z0, zl).
-inline int face_pass_mask(const StepPlan& p) {
+inline int face_pass_mask(const StepPlan& p, int bytes) {
   int m = 0;
   for (int o = 0; o < p.nops; o++) {
     const PlaneOp& op = p.ops[o];
-    if (op.kind == OP_POST_BB) {
+    if (op.kind == OP_POST_BB || (op.kind == OP_CAVITY && bytes == 2)) {
       for (int f = 0; f < 6; f++)
         if (!p.periodic[f / 2]) m |= 1 << f;
+    } else if (op.kind == OP_CAVITY) {
+      for (int f = 4; f < 6; f++)
+        if (p.ncav[f] > 0) m |= 1 << f;
     } else if (op.kind == OP_ZOUHE || op.kind == OP_LID) {
       m |= 1 << op.face;
     }

@@ -142,6 +142,15 @@ template <typename S>
 __device__ __forceinline__ S ld_stream(const S* p) {
   return __ldg(p);
 }
+// A population read. LIVE: the lattice is written by other SMs inside this launch (the resident
+// kernel), so the read goes to L2.
+template <bool LIVE, typename S>
+__device__ __forceinline__ S ld_pop(const S* p) {
+  if constexpr (LIVE)
+    return __ldcg(p);
+  else
+    return ld_stream(p);
+}
 
 // ------------------------------------------------------------------ storage rounding
 // With 16-bit storage a round-to-nearest store loses every update smaller than half a storage
@@ -753,7 +762,7 @@ __device__ __forceinline__ bool on_face(int x, int y, int z, const StepPlan& p) 
 // post_bounce_back over the non-periodic faces in launcher order x0, xl, y0, yl, z0, zl
 // (post_bounce_back.cu:115-120): the value saved by pre_bounce_back is this node's own
 // post-collision opposite population, plus the cavity increments of that face.
-template <typename S, typename R>
+template <typename S, typename R, bool LIVE>
 __device__ __forceinline__ void post_bb(R (&v)[Q], const S* __restrict__ fin, int64_t idx, int x, int y, int z,
                                         const StepPlan& p) {
   Unroll<0, 6>::run([&]<int F>() {
@@ -761,10 +770,24 @@ __device__ __forceinline__ void post_bb(R (&v)[Q], const S* __restrict__ fin, in
     if (!on_face<F>(x, y, z, p)) return;
     Unroll<0, 5>::run([&]<int K>() {
       constexpr int dst = PlaneBB::post[F][K], src = PlaneBB::pre[F][K];
-      R val = Codec<S, R>::template dec<src>(ld_stream(fin + src * p.stride + idx), p);
+      R val = Codec<S, R>::template dec<src>(ld_pop<LIVE>(fin + src * p.stride + idx), p);
       for (int c = 0; c < p.ncav[F]; c++) val = val + R(p.cav[F][c][K]);
       v[dst] = val;
     });
+  });
+}
+
+// The cavity increments of a leading post_bounce_back (OP_CAVITY): the pulled values are the ones
+// it restores, so each increment adds to the value in hand.
+template <typename R>
+__device__ __forceinline__ void cavity_increments(R (&v)[Q], int z, const StepPlan& p) {
+  Unroll<4, 6>::run([&]<int F>() {
+    if (p.periodic[2] || z != (F == 4 ? 0 : p.nz - 1)) return;
+    for (int c = 0; c < p.ncav[F]; c++)
+      Unroll<0, 5>::run([&]<int K>() {
+        constexpr int dst = PlaneBB::post[F][K];
+        v[dst] = v[dst] + R(p.cav[F][c][K]);
+      });
   });
 }
 
@@ -813,13 +836,17 @@ __device__ __forceinline__ void zero_gradient_node(S* __restrict__ fin, const in
   });
 }
 
-template <typename S, typename R>
+template <typename S, typename R, bool LIVE>
 __device__ __forceinline__ void plane_ops(R (&v)[Q], const S* __restrict__ fin, int64_t idx, int x, int y, int z,
                                           int8_t flag, const StepPlan& p) {
   for (int o = 0; o < p.nops; o++) {
     const PlaneOp& op = p.ops[o];
     if (op.kind == OP_POST_BB) {
-      post_bb<S, R>(v, fin, idx, x, y, z, p);
+      post_bb<S, R, LIVE>(v, fin, idx, x, y, z, p);
+      continue;
+    }
+    if (op.kind == OP_CAVITY) {
+      cavity_increments<R>(v, z, p);
       continue;
     }
     if (op.kind == OP_ZERO_GRADIENT) continue;  // applied by the outlet pass before the step
@@ -961,13 +988,13 @@ __device__ __forceinline__ bool on_op_z_face(const StepPlan& p, int z) {
 // (`pulled` false for a first step, which collides the initial state), start_iteration boxes,
 // collision.  The 16-bit tiers carry scaled deviations; the boundary operators and the boxes work
 // on full populations, so those nodes convert around them.
-template <typename S, typename R, bool STRICT, int MODE, int COLL>
+template <typename S, typename R, bool STRICT, int MODE, int COLL, bool LIVE = false>
 __device__ __forceinline__ void node_update(R (&v)[Q], const S* __restrict__ fin, int64_t idx, int x, int y, int z,
                                             int8_t flag, const StepPlan& p, bool pulled, bool edge) {
   constexpr bool DEV = is_16bit<S>();
   if (pulled && edge && p.nops > 0) {
     if constexpr (DEV) Unroll<0, Q>::run([&]<int I>() { v[I] = fmaf(v[I], R(p.inv_scale), R(p.dref[I])); });
-    plane_ops<S, R>(v, fin, idx, x, y, z, flag, p);
+    plane_ops<S, R, LIVE>(v, fin, idx, x, y, z, flag, p);
     if constexpr (DEV) Unroll<0, Q>::run([&]<int I>() { v[I] = (v[I] - R(p.dref[I])) * R(p.scale); });
   }
   if (MODE != MODE_FINISH) {
@@ -996,9 +1023,10 @@ __device__ __forceinline__ void pair_update(float2 (&v)[Q], const StepPlan& p, i
     Unroll<0, Q>::run([&]<int I>() { v[I] = Lanes<float2>::select(wall, Lanes<float2>::splat(wall_value<S, I>(p)), v[I]); });
 }
 
-template <typename S, bool WALLS>
+template <typename S, bool WALLS, bool LIVE>
 __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
-                                          const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q]);
+                                          const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
+                                          bool walls);
 
 // The stored values the node (x, y, z) gathers (pull with periodic wrap and on-node bounce-back;
 // in the prologue its own values), every load issued before any is used.  A bounced value (the
@@ -1009,15 +1037,17 @@ __device__ __forceinline__ void node_gather(const S* __restrict__ fin, const int
   if constexpr (MODE == MODE_PROLOGUE) {
     Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_stream(fin + I * p.stride + idx); });
   } else {
-    node_pull<S, WALLS>(fin, flags, p, x, y, z, idx, raw);
+    node_pull<S, WALLS, false>(fin, flags, p, x, y, z, idx, raw, true);
   }
 }
 
 // node_gather's pull: source coordinates x - e for e in {+1, 0, -1}; periodic axes wrap, others
-// flag "outside" (on-node bounce-back), as do wall sources where wall_bounce_back is active.
-template <typename S, bool WALLS>
+// flag "outside" (on-node bounce-back), as do wall sources where wall_bounce_back is active (WALLS
+// and, in kernels that take several plans, `walls`).
+template <typename S, bool WALLS, bool LIVE>
 __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
-                                          const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q]) {
+                                          const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
+                                          bool walls) {
   int sx[3], sy[3], sz[3];
   bool ox[3], oy[3], oz[3];
 #pragma unroll
@@ -1039,14 +1069,14 @@ __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_
     sz[k] = cz;
   }
   bool near = true;  // whether some pull may come from a wall node
-  if constexpr (WALLS) near = p.nearwall == nullptr || p.nearwall[idx] != 0;
+  if constexpr (WALLS) near = walls && (p.nearwall == nullptr || p.nearwall[idx] != 0);
   Unroll<0, Q>::run([&]<int I>() {
     constexpr int kx = 1 - D3Q19::ex[I], ky = 1 - D3Q19::ey[I], kz = 1 - D3Q19::ez[I];
     constexpr int O = D3Q19::opp(I);
     bool bounce = ox[kx] || oy[ky] || oz[kz];
     const int64_t src = ((int64_t)sz[kz] * p.ny + sy[ky]) * p.nx + sx[kx];
     if (WALLS && I != 0 && !bounce && near) bounce = (flags[src] == FLAG_WALL);
-    raw[I] = ld_stream(bounce ? fin + O * p.stride + idx : fin + I * p.stride + src);
+    raw[I] = ld_pop<LIVE>(bounce ? fin + O * p.stride + idx : fin + I * p.stride + src);
   });
 }
 
