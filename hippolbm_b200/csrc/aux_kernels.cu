@@ -398,7 +398,7 @@ cudaError_t launch_rasterize(int8_t* flags, const StepPlan& p, const int lo[3], 
   return cudaGetLastError();
 }
 
-// near[idx] = 1 when a direction of node idx pulls from a wall node (the pull the step kernels
+// near[idx] = 2 for a wall node, else 1 when a direction of node idx pulls from a wall node (the pull the step kernels
 // replace by on-node bounce-back under wall_bounce_back), with the gather's periodic wrap; pulls
 // from outside a non-periodic face bounce anyway and are not counted.
 __global__ void k_near_wall(const int8_t* __restrict__ flags, int8_t* __restrict__ near, int nx, int ny, int nz,
@@ -417,7 +417,28 @@ __global__ void k_near_wall(const int8_t* __restrict__ flags, int8_t* __restrict
         if (sz < 0 || sz >= nz) { if (!pz) continue; sz = sz < 0 ? sz + nz : sz - nz; }
         if (flags[(int64_t(sz) * ny + sy) * nx + sx] == FLAG_WALL) any = 1;
       }
-  near[(int64_t(z) * ny + y) * nx + x] = any;
+  const int64_t idx = (int64_t(z) * ny + y) * nx + x;
+  near[idx] = flags[idx] == FLAG_WALL ? 2 : any;
+}
+
+// Counts the near-wall nodes or, with `list`, writes them down: one atomic per warp, so the nodes of
+// a warp stay together.
+__global__ void k_near_list(const int8_t* __restrict__ near, int64_t ncell, int32_t* counter, uint32_t* list) {
+  const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool hit = idx < ncell && near[idx] == 1;
+  const unsigned m = __ballot_sync(0xffffffffu, hit);
+  if (m == 0) return;
+  const int lane = threadIdx.x & 31;
+  int base = 0;
+  if (lane == 0) base = atomicAdd(counter, __popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (hit && list) list[base + __popc(m & ((1u << lane) - 1u))] = uint32_t(idx);
+}
+
+cudaError_t launch_near_list(const int8_t* near, int64_t ncell, int32_t* counter, uint32_t* list, cudaStream_t s) {
+  if (cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int32_t), s)) return e;
+  k_near_list<<<unsigned((ncell + 255) / 256), 256, 0, s>>>(near, ncell, counter, list);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_near_wall(const int8_t* flags, int8_t* near, const int n[3], const int periodic[3],

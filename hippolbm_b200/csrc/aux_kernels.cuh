@@ -25,6 +25,8 @@ cudaError_t launch_rasterize(int8_t* flags, const StepPlan& p, const int lo[3], 
                              const ObstacleDesc& o, cudaStream_t s);
 cudaError_t launch_near_wall(const int8_t* flags, int8_t* near, const int n[3], const int periodic[3],
                              cudaStream_t s);
+// *counter = nodes with near == 1; with `list`, those nodes (the nodes of a warp in order)
+cudaError_t launch_near_list(const int8_t* near, int64_t ncell, int32_t* counter, uint32_t* list, cudaStream_t s);
 int stats_blocks(int64_t ncell);
 cudaError_t launch_macro_stats(int prec, const void* f, const int8_t* flags, const StepPlan& p, double* rho,
                                double* u, double* partials, double* out3, cudaStream_t s);

@@ -124,7 +124,10 @@ struct hlbm_ctx {
   void* f[2] = {nullptr, nullptr};
   int cur = 0;
   int8_t* flags = nullptr;
-  int8_t* nearwall = nullptr;  // per node: some pull comes from a wall node (k_near_wall)
+  int8_t* nearwall = nullptr;  // per node: 1 some pull comes from a wall node, 2 a wall node (k_near_wall)
+  uint32_t* near_list = nullptr;  // the nodes marked 1, for plans with wall_bounce_back; built with the plan
+  int32_t near_count = 0;
+  bool near_stale = true;         // the map changed after the list was built
   bool maybe_walls = false;     // the flags may hold wall nodes (an obstacle was rasterised or put)
   bool variant_tuned = false;   // hlbm_tune / hlbm_autotune chose the variant (else the tier default)
   bool variant_forced = false;  // hlbm_tune chose it: the step kernel of that variant runs, never the resident one
@@ -198,7 +201,36 @@ void storage_reference(const hlbm_ctx* c, float dref[Q]) {
 // the near-wall map after the flags changed (stream-ordered after the change)
 int refresh_near_wall(hlbm_ctx* c) {
   c->launches++;
+  c->near_stale = true;
+  c->plan_dirty = true;
   HLBM_CK(launch_near_wall(c->flags, c->nearwall, c->n, c->periodic, c->stream));
+  return HLBM_OK;
+}
+
+// The list of the near-wall nodes (k_near_list), which the fix-up walks: a sphere of radius
+// 20 leaves 7 k of 2.4 M nodes to look at.  Counted, allocated and filled when a
+// plan with wall_bounce_back is built after the flags changed.
+int refresh_near_list(hlbm_ctx* c) {
+  if (!c->near_stale) return HLBM_OK;
+  pool_free(c->near_list, c->stream);
+  c->near_list = nullptr;
+  c->near_count = 0;
+  int32_t* counter = reinterpret_cast<int32_t*>(c->stats_dev);
+  c->launches++;
+  HLBM_CK(launch_near_list(c->nearwall, c->ncell, counter, nullptr, c->stream));
+  int32_t n = 0;
+  HLBM_CK(cudaMemcpyAsync(&n, counter, sizeof(n), cudaMemcpyDeviceToHost, c->stream));
+  HLBM_CK(cudaStreamSynchronize(c->stream));
+  if (n > 0) {
+    if (pool_alloc((void**)&c->near_list, size_t(n) * sizeof(uint32_t), c->device, c->stream) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(HLBM_ENOMEM, "cannot allocate the list of near-wall nodes");
+    }
+    c->launches++;
+    HLBM_CK(launch_near_list(c->nearwall, c->ncell, counter, c->near_list, c->stream));
+  }
+  c->near_count = n;
+  c->near_stale = false;
   return HLBM_OK;
 }
 
@@ -212,6 +244,7 @@ void base_plan(hlbm_ctx* c, StepPlan& p) {
   p.stride = c->stride;
   p.rho0 = c->rho0;
   p.nearwall = c->nearwall;
+  p.overlap = 1;
   p.wall_flags = c->maybe_walls ? 1 : 0;
   p.scale = c->scale;
   p.inv_scale = 1.0 / c->scale;
@@ -386,6 +419,11 @@ int build_plan(hlbm_ctx* c) {
     b.value = h.value;
   }
   p.face_mask = face_pass_mask(p, int(elem_size(c->precision)));
+  if (p.walls && p.wall_flags && p.ncell <= int64_t(0xffffffffu)) {
+    if (int rc = refresh_near_list(c)) return rc;
+    p.near_list = c->near_list;
+    p.near_count = c->near_count;
+  }
   if (int rc = setup_pipeline(c)) return rc;
   c->plan_dirty = false;
   c->plan_version++;
@@ -480,15 +518,17 @@ cudaError_t launch_with_plan(hlbm_ctx* c, int mode, const void* fin, void* fout,
   t.sms = c->sms;
   const int bytes = int(elem_size(c->precision));
   c->launches++;
-  if (rows_runs(p, variant, mode, bytes)) {  // the row pipeline, then the face pass and the wall fix-up
-    if (p.face_mask != 0) c->launches++;
-    if (walls) c->launches++;
-  } else {
-    if (variant >= 8) variant = 5;  // what launch_step runs for variants 8 and 9 here
-    if (face_pass_runs(p, walls, variant, mode == MODE_PROLOGUE, bytes))
-      c->launches++;  // the face pass after the step kernel
-    if (walls && mode != MODE_PROLOGUE && variant < 6 && variant % 2 == 1 && vec_eligible_bytes(p, walls, bytes, variant))
-      c->launches++;  // the wall fix-up after the vectorised kernel
+  if (mode == MODE_FUSED) {  // the fix-up after the step kernel
+    int v = variant;
+    const bool rows = rows_runs(p, v, mode, bytes);
+    if (v >= 8 && !rows) v = 5;  // what launch_step runs for variants 8 and 9 here
+    const bool vec = v < 6 && v % 2 == 1 && vec_eligible_bytes(p, walls, bytes, v);
+    const bool face_pass = rows || vec || (v < 6 && bytes < 8);
+    if ((face_pass && p.face_mask != 0) || (walls && (rows || vec) && p.near_count > 0)) c->launches++;
+  } else if (mode == MODE_FINISH) {
+    if (variant >= 8) variant = 5;
+    if (face_pass_runs(p, walls, variant, false, bytes)) c->launches++;
+    if (walls && variant < 6 && variant % 2 == 1 && vec_eligible_bytes(p, walls, bytes, variant)) c->launches++;
   }
   switch (c->precision) {
     case HLBM_F64: return step_f64(mode, walls, fin, fout, c->flags, p, s, variant, t);
@@ -660,7 +700,7 @@ int hlbm_destroy(hlbm_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) {  // the memory returns to the pool once the stream's work is done
     void* bufs[] = {c->f[0], c->f[1], c->flags, c->nearwall, c->partials, c->stats_dev, c->plane_tmp, c->uprev,
-                    c->plan_dev, c->desc_dev, c->tiles_dev, c->err_dev, c->seed_dev, c->group_dev};
+                    c->plan_dev, c->desc_dev, c->tiles_dev, c->err_dev, c->seed_dev, c->group_dev, c->near_list};
     for (void* b : bufs) pool_free(b, c->stream);
     cudaStreamDestroy(c->stream);
   }
@@ -1396,6 +1436,7 @@ int batch_capture_concurrent(hlbm_batch* b) {
       StepPlan pk = c->plan;
       pk.seed_dev = sr ? c->seed_dev : nullptr;
       pk.seed_parity = k;
+      pk.overlap = 0;
       e = launch_with_plan(c, MODE_FUSED, c->f[c->cur ^ k], c->f[c->cur ^ k ^ 1], pk, concurrent_variant(c), c->stream);
     }
     if (e == cudaSuccess) e = cudaEventRecord(c->join_ev, c->stream);
@@ -1788,9 +1829,11 @@ int hlbm_batch_autotune(hlbm_batch* b, int32_t reps, int32_t* chosen, double* ms
       for (hlbm_ctx* c : b->members) {
         if (e == cudaSuccess && !c->join_ev) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, b->fork_ev, 0);
+        StepPlan pk = c->plan;
+        pk.overlap = 0;
         if (e == cudaSuccess)
           e = launch_with_plan(c, c->phase == RAW ? MODE_PROLOGUE : MODE_FUSED, c->f[c->cur], c->f[1 - c->cur],
-                               c->plan, concurrent_variant(c), c->stream);
+                               pk, concurrent_variant(c), c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(c->join_ev, c->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, c->join_ev, 0);
       }

@@ -76,6 +76,7 @@ struct StepPlan {
   // when set, the step number comes from seed_dev[seed_parity] instead of `seed`, and the launch
   // writes seed_dev[seed_parity ^ 1] = that + 1 (launches replayed from a captured graph)
   uint32_t* seed_dev;
+  int32_t overlap;  // step launches may start while the launch before them drains (never in captured graphs)
   int32_t seed_parity;
   // geometry of the one-node-per-thread kernel: 0 = x on threadIdx.x, y on threadIdx.y (rows of
   // whole warps); 1 = blocks of 256 consecutive nodes of a z-plane, for rows that would leave
@@ -83,11 +84,14 @@ struct StepPlan {
   int32_t linear;
   float inv_nx;
   int32_t face_mask;  // face_pass_mask of the plan: faces whose nodes the boundary operators change
-  // per node: 1 when some direction pulls from a wall node (k_near_wall); nodes with 0 skip the
-  // wall test of every pull.  Null: test every pull.
+  // per node: 1 when some direction pulls from a wall node, 2 for a wall node (k_near_wall); nodes
+  // with 0 skip the wall test of every pull.  Null: test every pull.
   const int8_t* nearwall;
   // the flags may hold wall nodes (an obstacle was rasterised or wall flags were put)
   int32_t wall_flags;
+  // the near-wall nodes (nearwall == 1), while wall_bounce_back is active; null: no list
+  const uint32_t* near_list;
+  int32_t near_count;
   PlaneOp ops[MAX_PLANE_OPS];
   SetBox sets[MAX_SETS];
 };

@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "lbm_step_rows.cuh"
 #include "lbm_step_spans.cuh"
 #include "lbm_step_tiles.cuh"
@@ -28,6 +30,32 @@ inline void step_geometry(const StepPlan& p, dim3& grid, dim3& block) {
   grid = dim3((p.nx + bx - 1) / bx, (p.ny + by - 1) / by, p.nz);
 }
 
+// A launch on stream s; with p.overlap it may start while the launch before it drains (pdl_wait).
+template <class... P, class... A>
+cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const StepPlan& p, cudaStream_t s, A&&... a) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = p.overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(a)...);
+}
+
+// The fix-up after a fused step kernel (k_fixup); nothing when no node needs it.
+template <typename S, typename R, bool STRICT, bool WALLS>
+cudaError_t launch_fixup(const S* fi, S* fo, const int8_t* flags, const StepPlan& p, bool list, cudaStream_t s) {
+  const FixGeometry g = fix_geometry(p, list);
+  if (g.total == 0) return cudaSuccess;
+  const dim3 grid((g.total + FIX_THREADS - 1) / FIX_THREADS);
+  if (p.collision == 0) return launch_kernel(k_fixup<S, R, STRICT, WALLS, 0>, grid, dim3(FIX_THREADS), 0, p, s, fi, fo, flags, p, g);
+  return launch_kernel(k_fixup<S, R, STRICT, WALLS, 1>, grid, dim3(FIX_THREADS), 0, p, s, fi, fo, flags, p, g);
+}
+
 // The face pass after a step kernel that left the boundary operators out: the nodes of the faces
 // in p.face_mask, recomputed whole by the one-node step.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS>
@@ -42,12 +70,8 @@ cudaError_t launch_faces(const S* fi, S* fo, const int8_t* flags, const StepPlan
     }
   if ((faces & 3) == 3 && 2 * int64_t(p.ny) * p.nz > area) area = 2 * int64_t(p.ny) * p.nz;  // x faces interleaved
   const dim3 fgrid(unsigned((area + 255) / 256), 6, 1);
-  if (MODE == MODE_FUSED && p.collision == 0)
-    k_faces<S, R, STRICT, MODE, WALLS, 0><<<fgrid, 256, 0, s>>>(fi, fo, flags, p, faces);
-  else if (MODE == MODE_FUSED)
-    k_faces<S, R, STRICT, MODE, WALLS, 1><<<fgrid, 256, 0, s>>>(fi, fo, flags, p, faces);
-  else
-    k_faces<S, R, STRICT, MODE, WALLS, 2><<<fgrid, 256, 0, s>>>(fi, fo, flags, p, faces);
+  if constexpr (MODE == MODE_FUSED) return launch_fixup<S, R, STRICT, WALLS>(fi, fo, flags, p, false, s);
+  k_faces<S, R, STRICT, MODE, WALLS, 2><<<fgrid, 256, 0, s>>>(fi, fo, flags, p, faces);
   return cudaGetLastError();
 }
 
@@ -61,23 +85,23 @@ cudaError_t launch_one(const void* fin, void* fout, const int8_t* flags, const S
     if (pairs_eligible(p)) {  // two nodes per thread, packed stores
       const int64_t plane = int64_t(p.nx) * p.ny;
       const dim3 pgrid(unsigned((plane / 2 + 255) / 256), p.nz, 1);
-      if (MODE == MODE_FUSED && p.collision == 0)
-        k_step_pairs<S, R, STRICT, MODE, WALLS, 0, MINB><<<pgrid, 256, 0, s>>>(fi, fo, flags, p);
-      else if (MODE == MODE_FUSED)
-        k_step_pairs<S, R, STRICT, MODE, WALLS, 1, MINB><<<pgrid, 256, 0, s>>>(fi, fo, flags, p);
+      constexpr bool FUSED = MODE == MODE_FUSED;
+      cudaError_t e;
+      if (FUSED && p.collision == 0)
+        e = launch_kernel(k_step_pairs<S, R, STRICT, MODE, WALLS, FUSED ? 0 : 2, MINB>, pgrid, dim3(256), 0, p, s, fi, fo, flags, p);
       else
-        k_step_pairs<S, R, STRICT, MODE, WALLS, 2, MINB><<<pgrid, 256, 0, s>>>(fi, fo, flags, p);
-      if (cudaError_t e = cudaGetLastError()) return e;
+        e = launch_kernel(k_step_pairs<S, R, STRICT, MODE, WALLS, FUSED ? 1 : 2, MINB>, pgrid, dim3(256), 0, p, s, fi, fo, flags, p);
+      if (e) return e;
       return launch_faces<S, R, STRICT, MODE, WALLS>(fi, fo, flags, p, s);
     }
   }
-  if (MODE == MODE_FUSED && p.collision == 0)
-    k_step<S, R, STRICT, MODE, WALLS, 0, MINB><<<grid, block, 0, s>>>(fi, fo, flags, p);
-  else if (MODE == MODE_FUSED)
-    k_step<S, R, STRICT, MODE, WALLS, 1, MINB><<<grid, block, 0, s>>>(fi, fo, flags, p);
+  constexpr bool FUSED = MODE == MODE_FUSED;
+  cudaError_t e;
+  if (FUSED && p.collision == 0)
+    e = launch_kernel(k_step<S, R, STRICT, MODE, WALLS, FUSED ? 0 : 2, MINB>, grid, block, 0, p, s, fi, fo, flags, p);
   else
-    k_step<S, R, STRICT, MODE, WALLS, 2, MINB><<<grid, block, 0, s>>>(fi, fo, flags, p);
-  if (cudaError_t e = cudaGetLastError()) return e;
+    e = launch_kernel(k_step<S, R, STRICT, MODE, WALLS, FUSED ? 1 : 2, MINB>, grid, block, 0, p, s, fi, fo, flags, p);
+  if (e) return e;
   if constexpr (face_pass_tier<S>()) return launch_faces<S, R, STRICT, MODE, WALLS>(fi, fo, flags, p, s);
   return cudaSuccess;
 }
@@ -107,22 +131,19 @@ cudaError_t launch_vec(int walls, const void* fin, void* fout, const int8_t* fla
   const S* fi = static_cast<const S*>(fin);
   S* fo = static_cast<S*>(fout);
   const Planes<S> pl = make_planes(fi, fo, p.stride);
-  if (MODE == MODE_FUSED && p.collision == 0)
-    k_step_vec<S, R, STRICT, MODE, NPT, 0, MINB><<<grid, block, 0, s>>>(pl, flags, p);
-  else if (MODE == MODE_FUSED)
-    k_step_vec<S, R, STRICT, MODE, NPT, 1, MINB><<<grid, block, 0, s>>>(pl, flags, p);
+  constexpr bool FUSED = MODE == MODE_FUSED;
+  cudaError_t e;
+  if (FUSED && p.collision == 0)
+    e = launch_kernel(k_step_vec<S, R, STRICT, MODE, NPT, FUSED ? 0 : 2, MINB>, grid, block, 0, p, s, pl, flags, p);
   else
-    k_step_vec<S, R, STRICT, MODE, NPT, 2, MINB><<<grid, block, 0, s>>>(pl, flags, p);
-  if (cudaError_t e = cudaGetLastError()) return e;
-  if (cudaError_t e = launch_faces<S, R, STRICT, MODE, false>(fi, fo, flags, p, s)) return e;
-  if (!walls || MODE == MODE_PROLOGUE) return cudaSuccess;
-  const unsigned wgrid = unsigned((p.ncell + 255) / 256);
-  if (MODE == MODE_FUSED && p.collision == 0)
-    k_wall_fixup<S, R, STRICT, MODE, 0><<<wgrid, 256, 0, s>>>(fi, fo, flags, p);
-  else if (MODE == MODE_FUSED)
-    k_wall_fixup<S, R, STRICT, MODE, 1><<<wgrid, 256, 0, s>>>(fi, fo, flags, p);
-  else
-    k_wall_fixup<S, R, STRICT, MODE, 2><<<wgrid, 256, 0, s>>>(fi, fo, flags, p);
+    e = launch_kernel(k_step_vec<S, R, STRICT, MODE, NPT, FUSED ? 1 : 2, MINB>, grid, block, 0, p, s, pl, flags, p);
+  if (e || MODE == MODE_PROLOGUE) return e;
+  if constexpr (FUSED)
+    return walls ? launch_fixup<S, R, STRICT, true>(fi, fo, flags, p, true, s)
+                 : launch_fixup<S, R, STRICT, false>(fi, fo, flags, p, false, s);
+  if ((e = launch_faces<S, R, STRICT, MODE, false>(fi, fo, flags, p, s))) return e;
+  if (!walls) return cudaSuccess;
+  k_wall_fixup<S, R, STRICT, MODE, 2><<<unsigned((p.ncell + 255) / 256), 256, 0, s>>>(fi, fo, flags, p);
   return cudaGetLastError();
 }
 
@@ -244,8 +265,7 @@ cudaError_t launch_rows_t(const Planes<S>& pl, const int8_t* flags, const StepPl
   const size_t smem = rows_smem_bytes(STAGES, g);
   if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return e;
   const int grid = g.ntiles < a.sms * MINB ? g.ntiles : a.sms * MINB;
-  kern<<<grid, 32 * (WARPS + 1), smem, s>>>(pl, flags, p, g, a.err, a.wait_limit);
-  return cudaGetLastError();
+  return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, pl, flags, p, g, a.err, a.wait_limit);
 }
 
 template <typename S, int COLL, int WARPS, int MINB>
@@ -276,8 +296,7 @@ cudaError_t launch_spans_t(const Planes<S>& pl, const int8_t* flags, const StepP
   const size_t smem = spans_smem_bytes(STAGES, g);
   if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return e;
   const int grid = g.ntiles < a.sms * MINB ? g.ntiles : a.sms * MINB;
-  kern<<<grid, 32 * (WARPS + 1), smem, s>>>(pl, flags, p, g, a.err, a.wait_limit);
-  return cudaGetLastError();
+  return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, pl, flags, p, g, a.err, a.wait_limit);
 }
 
 // Which pipeline a fused step of `variant` (8 or 9) runs on the lattice: 1 the row pipeline (rows
@@ -320,14 +339,8 @@ cudaError_t launch_rows(int mode, int walls, const void* fin, void* fout, const 
         e = p.collision == 0 ? launch_spans_t<S, 0, 9>(pl, flags, p, g, a, s) : launch_spans_t<S, 1, 9>(pl, flags, p, g, a, s);
     }
     if (e) return e;
-    if ((e = launch_faces<S, R, STRICT, MODE_FUSED, false>(fi, fo, flags, p, s))) return e;
-    if (!walls) return cudaSuccess;
-    const unsigned wgrid = unsigned((p.ncell + 255) / 256);
-    if (p.collision == 0)
-      k_wall_fixup<S, R, STRICT, MODE_FUSED, 0><<<wgrid, 256, 0, s>>>(fi, fo, flags, p);
-    else
-      k_wall_fixup<S, R, STRICT, MODE_FUSED, 1><<<wgrid, 256, 0, s>>>(fi, fo, flags, p);
-    return cudaGetLastError();
+    return walls ? launch_fixup<S, R, STRICT, true>(fi, fo, flags, p, true, s)
+                 : launch_fixup<S, R, STRICT, false>(fi, fo, flags, p, false, s);
   }
 }
 

@@ -108,6 +108,9 @@ __device__ __forceinline__ S rows_edge_value(const S* row, int x, int nx, const 
                                              int xn, const StepPlan& p) {
   if (x >= 0 && x < nx) return row[x];
   if (p.periodic[0]) return row[x < 0 ? x + nx : x - nx];
+  // an operator face: the fix-up steps the node, any value does.  (Fetching the node's own one put ten
+  // dependent loads from global memory into every tile of a closed box.)
+  if (p.face_mask & (x < 0 ? 1 : 2)) return row[0];
   return ld_stream(pl.in[D3Q19::opp(I)] + own_row + uint32_t(xn));
 }
 
@@ -208,8 +211,8 @@ __device__ __forceinline__ void rows_read_interior(const S* row, int x0, uint32_
 
 template <typename S, int COLL, int STAGES, int WARPS, int MINB>
 __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
-    k_step_rows(const __grid_constant__ Planes<S> pl, const int8_t* __restrict__ flags, const StepPlan p,
-                RowsGeometry g, int* __restrict__ err, long long wait_limit) {
+    k_step_rows(const __grid_constant__ Planes<S> pl, const int8_t* __restrict__ flags, const __grid_constant__ StepPlan p,
+                const __grid_constant__ RowsGeometry g, int* __restrict__ err, long long wait_limit) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);
   uint64_t* empty = full + STAGES;
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_begin();
   advance_seed<S, MODE_FUSED>(p);
   __syncthreads();
 

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_begin();
   advance_seed<S, MODE_FUSED>(p);
   __syncthreads();
 

@@ -231,6 +231,7 @@ inline Planes<S> make_planes(const S* fin, S* fout, int64_t stride) {
 template <typename S, typename R, bool STRICT, int MODE, int NPT, int COLL, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_step_vec(const __grid_constant__ Planes<S> pl,
                                                      const int8_t* __restrict__ flags, const StepPlan p) {
+  pdl_begin();
   advance_seed<S, MODE>(p);
   const uint32_t seed = launch_seed<S>(p);
   const int tx = blockIdx.x * blockDim.x + threadIdx.x;  // vector index along x
