@@ -22,6 +22,7 @@
 #include "hippolbm.h"
 #include "launch.cuh"
 #include "lbm_step_resident.cuh"
+#include "observe.cuh"
 
 using namespace hlbm;
 
@@ -565,6 +566,19 @@ bool vec_applies(const hlbm_ctx* c, int variant) {
   return vec_eligible_bytes(c->plan, c->plan.walls, int(elem_size(c->precision)), variant);
 }
 
+// {sum rho, min |u|, max |u|} of S_k into stats_dev, from the post-collision state in fin
+cudaError_t observe_state(hlbm_ctx* c, const void* fin) {
+  const int blocks = stats_blocks(c->ncell);
+  unsigned* done = c->group_dev;  // zero between launches, like the many-step launches' counter
+  switch (c->precision) {
+    case HLBM_F64: return observe_f64(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F64_STRICT: return observe_f64_strict(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F32: return observe_f32(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F16: return observe_f16(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    default: return observe_bf16(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+  }
+}
+
 // make S_k available; returns the buffer holding it
 int state_buffer(hlbm_ctx* c, void** out) {
   if (int rc = check_device_error(c)) return rc;
@@ -1038,14 +1052,27 @@ int hlbm_macro_variables(hlbm_ctx* c, double* rho, double* u) {
 int hlbm_simulation_state(hlbm_ctx* c, double out[3]) {
   if (!c || !out) return fail(HLBM_EINVAL, "hlbm_simulation_state: NULL argument");
   if (int rc = set_device(c)) return rc;
-  void* s;
-  if (int rc = state_buffer(c, &s)) return rc;
-  StepPlan p;
-  base_plan(c, p);
-  c->launches += 2;
-  HLBM_CK(launch_macro_stats(c->precision, s, c->flags, p, nullptr, nullptr, c->partials, c->stats_dev, c->stream));
-  HLBM_CK(cudaMemcpyAsync(out, c->stats_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  if (c->phase == POSTCOL) {  // straight from the post-collision state; the idle buffer stays idle
+    if (int rc = build_plan(c)) return rc;
+    const void* fin = c->f[c->cur];
+    HLBM_CK(outlet_passes(c->precision, c->plan, c->desc_dev, 0, fin == c->f[0] ? 0 : 1, c->n, c->stream, c->launches));
+    c->launches++;
+    HLBM_CK(observe_state(c, fin));
+  } else {
+    const void* s = c->phase == RAW ? c->f[c->cur] : c->f[1 - c->cur];
+    StepPlan p;
+    base_plan(c, p);
+    c->launches += 2;
+    HLBM_CK(launch_macro_stats(c->precision, s, c->flags, p, nullptr, nullptr, c->partials, c->stats_dev, c->stream));
+  }
+  // the three numbers and the error word behind one wait for the stream
+  double h[4];
+  int e = 0;
+  HLBM_CK(cudaMemcpyAsync(&e, c->err_dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  HLBM_CK(cudaMemcpyAsync(h, c->stats_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   HLBM_CK(cudaStreamSynchronize(c->stream));
+  if (e != 0) return check_device_error(c);
+  for (int k = 0; k < 3; k++) out[k] = h[k];
   return HLBM_OK;
 }
 
