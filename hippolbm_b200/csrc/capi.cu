@@ -243,6 +243,8 @@ void base_plan(hlbm_ctx* c, StepPlan& p) {
   for (int d = 0; d < 3; d++) p.periodic[d] = c->periodic[d];
   p.ncell = c->ncell;
   p.stride = c->stride;
+  for (int i = 0; i < Q; i++)
+    p.pull[i] = i * p.stride - ((int64_t(D3Q19::ez[i]) * p.ny + D3Q19::ey[i]) * p.nx + D3Q19::ex[i]);
   p.rho0 = c->rho0;
   p.nearwall = c->nearwall;
   p.overlap = 1;
@@ -442,19 +444,16 @@ cudaError_t outlet_passes(int prec, const StepPlan& p, const LatticeDesc* descs,
   return cudaSuccess;
 }
 
-// Whether a lattice steps in the resident kernel (lbm_step_resident.cuh): both population buffers
-// together within this many bytes, a plan it takes, and no variant asked for by hlbm_tune.  Measured
-// (us a step, resident against one launch a step): FP64 24^3 3.0 / 6.3, 64^3 (80 MB) 14.1 / 14.5, 80^3
-// (156 MB) 40 / 30; FP32 24^3 2.6 / 11.4, 80^3 (78 MB) 17.2 / 24.9, 96^3 (134 MB) 42 / 39; FP16 24^3
-// 3.1 / 20.6, 80^3 (39 MB) 18.5 / 23.7, 96^3 (67 MB) 29.8 / 26.7 (the row pipeline copies in bulk).
-// 16-bit MRT keeps its step kernels: there the node-pair form of every kernel has to round alike.
-constexpr int64_t resident_bytes(int precision) {
-  return int64_t(precision == HLBM_F16 || precision == HLBM_BF16 ? 50 : 100) << 20;
-}
+// Whether a lattice steps in the resident kernel (lbm_step_resident.cuh): a plan it takes, no variant asked
+// for by hlbm_tune, and one node per thread of the GPU or, in the 16-bit tiers, both population buffers
+// within 50 MB.  Measured (us a step, resident against one launch a step): FP64 31^3 3.5 / 5.1, 48^3
+// 7.9 / 6.2; FP32 31^3 2.9 / 5.3, 48^3 6.2 / 6.2; FP16 31^3 3.8 / 15.2, 57 x 43 x 61 8.4 / 15.0, 80^3 (39 MB)
+// 18.1 / 16.9 couette and 18.0 / 34.6 cavity, 96^3 (67 MB) 29.8 / 21.9.  16-bit MRT keeps its step kernels:
+// there the node-pair form of every kernel has to round alike.
 bool resident_applies(const hlbm_ctx* c) {
   const bool half = elem_size(c->precision) == 2;
-  return !c->variant_forced && resident_plan(c->plan) && !(half && c->collision == 1) &&
-         2 * int64_t(Q) * c->ncell * int64_t(elem_size(c->precision)) <= resident_bytes(c->precision);
+  if (c->variant_forced || !resident_plan(c->plan) || (half && c->collision == 1)) return false;
+  return c->ncell <= int64_t(c->sms) * RES_THREADS || (half && 2 * int64_t(Q) * c->ncell * 2 <= int64_t(50) << 20);
 }
 
 cudaError_t launch_resident_tier(int precision, const ResidentArgs& a, int walls, cudaStream_t s) {

@@ -56,6 +56,7 @@ struct StepPlan {
   int32_t periodic[3];
   int64_t ncell;
   int64_t stride;  // elements between direction planes (>= ncell, padded)
+  int64_t pull[Q];  // where an inner node pulls direction I from: I * stride - d_I elements from its slot of plane 0
   int32_t collision;  // 0 BGK, 1 MRT
   int32_t walls;      // wall_bounce_back active
   int32_t has_force;

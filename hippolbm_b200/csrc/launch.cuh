@@ -114,9 +114,10 @@ constexpr int vec_npt() {
 
 inline void vec_geometry(const StepPlan& p, int npt, int block_x, dim3& grid, dim3& block) {
   const int nvec = p.nx / npt;
-  int bx = block_x > 0 ? block_x : 128;
-  const int rounded = ((nvec + 31) / 32) * 32;
-  if (rounded < bx) bx = rounded;
+  // whole warps in x, as many as divide the row's and leave 256 threads a block: 80 vectors (nx = 320 in
+  // FP32) as 3 warps of a row each would make blocks of 192 threads
+  const int warps = (nvec + 31) / 32;
+  const int bx = block_x > 0 ? block_x : 32 * (warps % 4 == 0 ? 4 : (warps % 2 == 0 ? 2 : 1));
   const int by = 256 / bx > 0 ? 256 / bx : 1;
   block = dim3(bx, by, 1);
   grid = dim3((nvec + bx - 1) / bx, (p.ny + by - 1) / by, p.nz);
@@ -252,15 +253,17 @@ cudaError_t launch_tiles(const TmaArgs& a, int walls, int variant, cudaStream_t 
 // The row pipeline (lbm_step_rows.cuh) for one lattice: variant 8 = two CTAs per SM, variant 9 =
 // one CTA per SM with deeper staging; the face pass and (with wall obstacles) the wall fix-up
 // follow.  Returns cudaErrorNotSupported when the lattice or the mode cannot take it.
-inline int rows_stages(const RowsGeometry& g, int ctas_per_sm) {
+constexpr int rows_stage_count(int warps, int ctas_per_sm) {
   const size_t budget = size_t(227 * 1024) / size_t(ctas_per_sm) - 1024;
-  const size_t fit = (budget - 128) / g.stage_bytes;
+  const size_t fit = (budget - 128) / rows_stage_bytes(warps);
   return fit >= 4 ? 4 : int(fit);
 }
 
-template <typename S, int COLL, int STAGES, int WARPS, int MINB>
-cudaError_t launch_rows_t(const Planes<S>& pl, const int8_t* flags, const StepPlan& p, const RowsGeometry& g,
-                          const TmaArgs& a, cudaStream_t s) {
+template <typename S, int COLL, int WARPS, int MINB>
+cudaError_t launch_rows_t(const Planes<S>& pl, const int8_t* flags, const StepPlan& p, const TmaArgs& a, cudaStream_t s) {
+  constexpr int STAGES = rows_stage_count(WARPS, MINB);
+  static_assert(STAGES >= 2, "row pipeline stages must fit");
+  const RowsGeometry g = rows_geometry(p, WARPS);
   auto kern = k_step_rows<S, COLL, STAGES, WARPS, MINB>;
   const size_t smem = rows_smem_bytes(STAGES, g);
   if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return e;
@@ -268,12 +271,12 @@ cudaError_t launch_rows_t(const Planes<S>& pl, const int8_t* flags, const StepPl
   return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, pl, flags, p, g, a.err, a.wait_limit);
 }
 
-template <typename S, int COLL, int WARPS, int MINB>
-cudaError_t launch_rows_stages(int stages, const Planes<S>& pl, const int8_t* flags, const StepPlan& p,
-                               const RowsGeometry& g, const TmaArgs& a, cudaStream_t s) {
-  if (stages >= 4) return launch_rows_t<S, COLL, 4, WARPS, MINB>(pl, flags, p, g, a, s);
-  if (stages == 3) return launch_rows_t<S, COLL, 3, WARPS, MINB>(pl, flags, p, g, a, s);
-  return launch_rows_t<S, COLL, 2, WARPS, MINB>(pl, flags, p, g, a, s);
+template <typename S, int COLL>
+cudaError_t launch_rows_variant(const Planes<S>& pl, const int8_t* flags, const StepPlan& p, const TmaArgs& a,
+                                cudaStream_t s, int variant) {
+  if (variant == 8) return launch_rows_t<S, COLL, rows_warps(8), rows_ctas_per_sm(8)>(pl, flags, p, a, s);
+  if (rows_wide(p)) return launch_rows_t<S, COLL, ROWS_WIDE_WARPS, 1>(pl, flags, p, a, s);
+  return launch_rows_t<S, COLL, rows_warps(9), 1>(pl, flags, p, a, s);
 }
 
 // The span pipeline (lbm_step_spans.cuh) with the shape of variant 8 or 9; its stage count is the
@@ -302,9 +305,7 @@ cudaError_t launch_spans_t(const Planes<S>& pl, const int8_t* flags, const StepP
 // Which pipeline a fused step of `variant` (8 or 9) runs on the lattice: 1 the row pipeline (rows
 // of whole 16-byte chunks), 2 the span pipeline (any other row length), 0 neither.
 inline int pipeline_kind(const StepPlan& p, int variant, int bytes) {
-  if (rows_eligible(p, bytes, rows_warps(variant)) &&
-      rows_stages(rows_geometry(p, bytes, rows_warps(variant)), rows_ctas_per_sm(variant)) >= 2)
-    return 1;
+  if (rows_eligible(p, bytes, rows_warps(variant))) return 1;
   if (spans_eligible(p, bytes)) return 2;
   return 0;
 }
@@ -322,15 +323,8 @@ cudaError_t launch_rows(int mode, int walls, const void* fin, void* fout, const 
     const Planes<S> pl = make_planes(fi, fo, p.stride);
     cudaError_t e;
     if (kind == 1) {
-      const int ctas = rows_ctas_per_sm(variant);
-      const RowsGeometry g = rows_geometry(p, int(sizeof(S)), rows_warps(variant));
-      const int stages = rows_stages(g, ctas);
-      if (variant == 8)
-        e = p.collision == 0 ? launch_rows_stages<S, 0, rows_warps(8), rows_ctas_per_sm(8)>(stages, pl, flags, p, g, a, s)
-                             : launch_rows_stages<S, 1, rows_warps(8), rows_ctas_per_sm(8)>(stages, pl, flags, p, g, a, s);
-      else
-        e = p.collision == 0 ? launch_rows_stages<S, 0, rows_warps(9), rows_ctas_per_sm(9)>(stages, pl, flags, p, g, a, s)
-                             : launch_rows_stages<S, 1, rows_warps(9), rows_ctas_per_sm(9)>(stages, pl, flags, p, g, a, s);
+      e = p.collision == 0 ? launch_rows_variant<S, 0>(pl, flags, p, a, s, variant)
+                           : launch_rows_variant<S, 1>(pl, flags, p, a, s, variant);
     } else {
       const SpansGeometry g = spans_geometry(p, rows_warps(variant));
       if (variant == 8)

@@ -1059,6 +1059,25 @@ template <typename S, bool WALLS, bool LIVE>
 __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls) {
+  if constexpr (!LIVE && sizeof(S) < 8) {
+    // A warp of inner nodes needs one constant offset per direction: about 250 instructions of index
+    // arithmetic less a node (the one-node FP32 step of a 181 x 150 x 170 channel is bound by issue).
+    // Decided per warp: lanes that went different ways would wait for each other's loads.  Measured (us a
+    // step): FP32 sphere 150 x 120 x 131 95 -> 84, Poiseuille 130 x 97 x 113 54 -> 51; FP64, bound by bytes,
+    // keeps the one path (sphere 124 -> 132 with two).
+    const bool inner = x > 0 && x < p.nx - 1 && y > 0 && y < p.ny - 1 && z > 0 && z < p.nz - 1;
+    if (__all_sync(__activemask(), inner)) {
+      const S* at = fin + idx;
+      Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<LIVE>(at + p.pull[I]); });
+      if constexpr (WALLS) {
+        if (walls && (p.nearwall == nullptr || p.nearwall[idx] != 0))
+          Unroll<1, Q>::run([&]<int I>() {
+            if (flags[idx + p.pull[I] - I * p.stride] == FLAG_WALL) raw[I] = ld_pop<LIVE>(at + D3Q19::opp(I) * p.stride);
+          });
+      }
+      return;
+    }
+  }
   int sx[3], sy[3], sz[3];
   bool ox[3], oy[3], oz[3];
 #pragma unroll

@@ -10,13 +10,14 @@
 // a lattice stepped alone is one task.  Measured (us a step): FP64 31^3 6.3 -> 3.5, FP32 24^3 11.4 ->
 // 2.6, FP16 24^3 20.6 -> 3.1, BF16 57 x 43 x 61 20 -> 8.4; the barrier alone takes 1.2 of them.
 //
-// Work of one step, in items of one thread, whole warps of one kind:
+// A lattice of no more nodes than the group has threads gets one node per thread for the whole launch,
+// whose addresses to pull from are computed once.  Larger ones (16-bit tiers) work through items, whole
+// warps of one kind:
 //   faces     the nodes on the lattice's faces, each once, by the general one-node gather (periodic
 //             wrap, on-node bounce-back) and the boundary operators;
-//   interior  nodes off the faces, whose sources are idx - d_I: one offset per direction, no index
-//             arithmetic per direction.  The 16-bit tiers take the node pairs (n, n + 1), n even, of
-//             every other kernel, in packed FP32 with one 32-bit store per direction (a pair with
-//             one node on a face stores its other half alone), so the stored bits are the same.
+//   interior  the node pairs (n, n + 1), n even, of every other kernel, whose sources are idx - d_I: one
+//             offset per direction, packed FP32 and one 32-bit store per direction (a pair with one node
+//             on a face stores its other half alone), so the stored bits are the same.
 // Warps are dealt out across the CTAs first, so a lattice of few items still uses every SM.
 //
 // The buffers change hands between SMs inside the launch, so populations are read past L1 (ld.cg);
@@ -73,7 +74,7 @@ struct ResidentGeometry {
   int off[Q];                      // element offset of direction I's source from the node's index
   uint32_t z_nodes, y_nodes, nface, nface_pad, nitems;  // face nodes in the z planes, then the y rows; all; padded
   uint32_t pair_begin;             // first pair's node: the last even index not above plane 1
-  uint64_t m_nx, m_plane, m_nxi, m_planei, m_yrow, m_ny2;
+  uint64_t m_nx, m_plane, m_yrow, m_ny2;
 };
 
 // pairs: the lattice runs node pairs (16-bit tiers, pair_kernels_apply); all_nodes: every node by
@@ -81,20 +82,16 @@ struct ResidentGeometry {
 __device__ inline void resident_geometry(const StepPlan& p, bool pairs, bool all_nodes, ResidentGeometry& g) {
   const uint32_t nx = p.nx, ny = p.ny, nz = p.nz;
   const uint32_t plane = nx * ny;
-  const uint32_t yi = ny - 2, zi = nz - 2, xi = nx - 2;  // every axis has at least two nodes
+  const uint32_t yi = ny - 2, zi = nz - 2;  // every axis has at least two nodes
   g.z_nodes = 2 * plane;
   g.y_nodes = 2 * nx * zi;
   g.nface = all_nodes ? uint32_t(p.ncell) : g.z_nodes + g.y_nodes + 2 * yi * zi;
   g.nface_pad = (g.nface + 31u) & ~31u;
   g.pair_begin = plane & ~1u;
-  uint32_t inner = xi * yi * zi;
-  if (pairs) inner = zi == 0 ? 0 : (uint32_t(p.ncell) - plane - g.pair_begin + 1) / 2;
-  if (all_nodes) inner = 0;
+  const uint32_t inner = !pairs || zi == 0 ? 0 : (uint32_t(p.ncell) - plane - g.pair_begin + 1) / 2;
   g.nitems = g.nface_pad + inner;
   g.m_nx = res_magic(nx);
   g.m_plane = res_magic(plane);
-  g.m_nxi = res_magic(xi);
-  g.m_planei = res_magic(uint64_t(xi) * yi);
   g.m_yrow = res_magic(2 * nx);
   g.m_ny2 = res_magic(2 * yi);
   Unroll<0, Q>::run([&]<int I>() {
@@ -154,27 +151,6 @@ __device__ __forceinline__ void resident_face(const S* fin, const int8_t* __rest
   it.idx = (uint32_t(it.z) * uint32_t(p.ny) + uint32_t(it.y)) * uint32_t(p.nx) + uint32_t(it.x);
   it.flag = flags[it.idx];
   node_pull<S, WALLS, true>(fin, flags, p, it.x, it.y, it.z, it.idx, raw, walls);
-}
-
-// The node of interior item i (counted on from the face items), and its stored values.
-template <typename S, bool WALLS>
-__device__ __forceinline__ void resident_inner(const S* fin, const int8_t* __restrict__ flags, const StepPlan& p,
-                                               const ResidentGeometry& g, bool walls, uint32_t i, ResidentNode& it,
-                                               S (&raw)[Q]) {
-  const uint32_t j = i - g.nface_pad;
-  const uint32_t k = res_div(j, g.m_planei), rem = j - k * uint32_t(p.nx - 2) * uint32_t(p.ny - 2);
-  const uint32_t r = res_div(rem, g.m_nxi);
-  it.z = int(k) + 1;
-  it.y = int(r) + 1;
-  it.x = int(rem - r * uint32_t(p.nx - 2)) + 1;
-  it.idx = (uint32_t(it.z) * uint32_t(p.ny) + uint32_t(it.y)) * uint32_t(p.nx) + uint32_t(it.x);
-  it.flag = flags[it.idx];
-  if (WALLS && walls && p.nearwall[it.idx] == 1) {
-    node_pull<S, WALLS, true>(fin, flags, p, it.x, it.y, it.z, it.idx, raw, walls);
-  } else {
-    const S* at = fin + it.idx;
-    Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<true>(at + g.off[I]); });
-  }
 }
 
 // The update and store of a fetched node (a wall node keeps its scratch).
@@ -322,7 +298,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
         }
         ok = step_done(k);
       }
-    } else {
+    } else if constexpr (is_16bit<S>()) {
       for (int k = 0; k < tk.nsteps && ok; k++) {
         const S* fin = static_cast<const S*>(L.f[cur0 ^ (k & 1)]);
         S* fout = static_cast<S*>(L.f[cur0 ^ (k & 1) ^ 1]);
@@ -331,31 +307,11 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
           if (i >= g.nface) continue;
           ResidentNode it;
           S raw[Q];
-          resident_face<S, WALLS>(fin, L.flags, p, g, walls, is_16bit<S>() && !pairs, i, it, raw);
+          resident_face<S, WALLS>(fin, L.flags, p, g, walls, !pairs, i, it, raw);
           resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, on_op_face(p, it.x, it.y, it.z));
         }
-        if constexpr (is_16bit<S>()) {
-          for (; i < g.nitems; i += nthreads)
-            resident_pair<S, WALLS>(fin, fout, L.flags, p, g, walls, g.pair_begin + 2 * (i - g.nface_pad));
-        } else {
-          constexpr bool AHEAD = sizeof(S) == 4;  // FP64: the next node's 19 values do not fit the registers
-          ResidentNode it;
-          S raw[Q];
-          if (AHEAD && i < g.nitems) resident_inner<S, WALLS>(fin, L.flags, p, g, walls, i, it, raw);
-          for (; i < g.nitems; i += nthreads) {
-            if constexpr (AHEAD) {  // the next node's values are on their way while this one collides
-              ResidentNode next;
-              S ahead[Q];
-              if (i + nthreads < g.nitems) resident_inner<S, WALLS>(fin, L.flags, p, g, walls, i + nthreads, next, ahead);
-              resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, false);
-              it = next;
-              Unroll<0, Q>::run([&]<int I>() { raw[I] = ahead[I]; });
-            } else {
-              resident_inner<S, WALLS>(fin, L.flags, p, g, walls, i, it, raw);
-              resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, false);
-            }
-          }
-        }
+        for (; i < g.nitems; i += nthreads)
+          resident_pair<S, WALLS>(fin, fout, L.flags, p, g, walls, g.pair_begin + 2 * (i - g.nface_pad));
         ok = step_done(k);
       }
     }

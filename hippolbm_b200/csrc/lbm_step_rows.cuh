@@ -37,6 +37,7 @@ constexpr int ROWS_NODES_PER_THREAD = 4;  // two node pairs
 // faster than 16 at 96.
 constexpr int rows_warps(int variant) { return variant == 8 ? 8 : 12; }
 constexpr int rows_ctas_per_sm(int variant) { return variant == 8 ? 2 : 1; }
+constexpr int ROWS_WIDE_WARPS = 15;
 constexpr int rows_tile_nodes(int warps) { return warps * 32 * ROWS_NODES_PER_THREAD; }
 
 // Geometry of the row pipeline for one lattice: `rows` per tile, stage bytes, tiles.
@@ -47,7 +48,8 @@ struct RowsGeometry {
   size_t stage_bytes = 0;  // 19 direction blocks of tile-node values (rows * nx used), then the flag bytes
 };
 
-inline size_t rows_align128(size_t b) { return (b + 127) / 128 * 128; }
+constexpr size_t rows_align128(size_t b) { return (b + 127) / 128 * 128; }
+constexpr size_t rows_stage_bytes(int warps) { return rows_align128(size_t(2 * Q + 1) * rows_tile_nodes(warps)); }
 
 // Whether a lattice can take the row pipeline: a 16-bit tier, rows of whole 16-byte chunks of flag
 // bytes (and so of populations) and no longer than a tile, 32-bit node offsets, and the pair
@@ -57,14 +59,26 @@ inline bool rows_eligible(const StepPlan& p, int bytes, int warps) {
          pair_kernels_apply(p, bytes);
 }
 
-inline RowsGeometry rows_geometry(const StepPlan& p, int bytes, int warps) {
+inline RowsGeometry rows_geometry(const StepPlan& p, int warps) {
   RowsGeometry g;
   g.rows = rows_tile_nodes(warps) / p.nx > 0 ? rows_tile_nodes(warps) / p.nx : 1;
   if (g.rows > p.ny) g.rows = p.ny;
   g.tiles_per_plane = (p.ny + g.rows - 1) / g.rows;
   g.ntiles = g.tiles_per_plane * p.nz;
-  g.stage_bytes = rows_align128(size_t(Q + 1) * rows_tile_nodes(warps) * bytes);
+  g.stage_bytes = rows_stage_bytes(warps);
   return g;
+}
+
+// Whether variant 9 takes 15 consumer warps, a tile of 1,920 nodes, instead of 12: where whole rows fill
+// its tile at least a tenth better.  Measured (us a step, 12 / 15 warps): nx = 320, 5/6 of the small tile and
+// all of the wide one, MRT 596 / 538 at 320^3; nx = 384, both full, BGK 246 / 255 and MRT 317 / 308 at
+// 384^2 x 128; nx = 512, full and 4/5, BGK 441 / 482.
+inline bool rows_wide(const StepPlan& p) {
+  const auto fill = [&](int warps) {
+    const int tile = rows_tile_nodes(warps), rows = tile / p.nx < p.ny ? tile / p.nx : p.ny;
+    return double(rows) * p.nx / tile;
+  };
+  return fill(ROWS_WIDE_WARPS) >= 1.1 * fill(rows_warps(9));
 }
 
 inline size_t rows_smem_bytes(int stages, const RowsGeometry& g) { return 128 + size_t(stages) * g.stage_bytes; }
