@@ -427,6 +427,9 @@ int build_plan(hlbm_ctx* c) {
     p.near_list = c->near_list;
     p.near_count = c->near_count;
   }
+  const int bytes = int(elem_size(c->precision));
+  if (!c->variant_tuned && bytes == 2)
+    c->variant = pipeline_kind(p, 9, bytes) == 2 && spans_avoided(p) ? 4 : 9;
   if (int rc = setup_pipeline(c)) return rc;
   c->plan_dirty = false;
   c->plan_version++;
@@ -999,6 +1002,11 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
   if (nsteps == 0) return HLBM_OK;
   if (int rc = set_device(c)) return rc;
   if (int rc = build_plan(c)) return rc;
+  // a caller's graph holds one plain launch a step: no cooperative launch, no overlapped ones
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  HLBM_CK(cudaStreamIsCapturing(c->stream, &capture));
+  const bool captured = capture != cudaStreamCaptureStatusNone;
+  c->plan.overlap = !captured;
   if (c->phase == MATER) c->phase = POSTCOL;
   if (c->phase == RAW) {
     HLBM_CK(launch_step_kernel(c, MODE_PROLOGUE, c->f[c->cur], c->f[1 - c->cur]));
@@ -1007,7 +1015,7 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
     c->steps++;
     nsteps--;
   }
-  if (nsteps > 0 && resident_applies(c)) return resident_steps(c, nsteps);
+  if (nsteps > 0 && !captured && resident_applies(c)) return resident_steps(c, nsteps);
   for (int64_t s = 0; s < nsteps; s++) {
     HLBM_CK(launch_step_kernel(c, MODE_FUSED, c->f[c->cur], c->f[1 - c->cur]));
     c->cur = 1 - c->cur;

@@ -98,12 +98,14 @@ struct StepPlan {
 };
 
 // Whether the kernels that update node pairs in packed FP32 (the vectorised kernel of the 4- and
-// 2-byte tiers, the 16-bit pair kernel) take a plan: no start_iteration boxes, no body force (the
-// force term would hold the pair's density in registers through the whole update), and wall nodes
-// only where wall_bounce_back makes their populations scratch (a pair collides both lanes).  Other
-// plans run the one-node kernel.
+// 2-byte tiers, the 16-bit pair kernel, the row and span pipelines) take a plan: no start_iteration
+// boxes, and wall nodes only where wall_bounce_back makes their populations scratch (a pair collides
+// both lanes).  Other plans run the one-node kernel, and so does 16-bit MRT with a body force, whose
+// pair form may round differently.  (With a body force a 96^3 FP16 lattice steps in 30 us by the one-node
+// kernel, 22 by the row pipeline.)
 inline bool pair_kernels_apply(const StepPlan& p, int bytes) {
-  return bytes == 8 || (p.nsets == 0 && !p.has_force && (!p.wall_flags || p.walls));
+  return bytes == 8 ||
+         (p.nsets == 0 && (!p.has_force || bytes == 4 || p.collision == 0) && (!p.wall_flags || p.walls));
 }
 
 // Nodes per thread of the vectorised step kernel for a storage type of `bytes` bytes: one 16-byte
@@ -127,6 +129,15 @@ inline bool vec_eligible_bytes(const StepPlan& p, int walls, int bytes, int vari
 inline bool pairs_eligible(const StepPlan& p) {
   const int64_t plane = int64_t(p.nx) * p.ny;
   return plane % 2 == 0 && plane < (int64_t(1) << 24) && pair_kernels_apply(p, 2);
+}
+
+// Whether a 16-bit lattice that the span pipeline would take (variant 9) steps by the pair kernel
+// (variant 4): where nodes on a face are no operator's, they gather all values from global memory in the span
+// kernel's consumers and stall its tiles.  Measured (us a step, spans / pairs): Couette 100 x 90 x 110 44 / 30,
+// 130 x 97 x 113 82 / 42, 181 x 150 x 170 311 / 111; closed box 181 x 150 x 170 113 / 134.  MRT only where the
+// pair form runs (even z-planes), so that the stored bits stay the pair form's.
+inline bool spans_avoided(const StepPlan& p) {
+  return p.face_mask != 0x3f && (p.collision == 0 || pairs_eligible(p));
 }
 
 // Whether a single-lattice launch of step variant `variant` (not the prologue) is followed by the

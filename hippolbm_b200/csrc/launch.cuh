@@ -30,9 +30,11 @@ inline void step_geometry(const StepPlan& p, dim3& grid, dim3& block) {
   grid = dim3((p.nx + bx - 1) / bx, (p.ny + by - 1) / by, p.nz);
 }
 
-// A launch on stream s; with p.overlap it may start while the launch before it drains (pdl_wait).
+// A launch on stream s; with p.overlap and `early` it may start while the launch before it drains
+// (pdl_wait).
 template <class... P, class... A>
-cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const StepPlan& p, cudaStream_t s, A&&... a) {
+cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const StepPlan& p, cudaStream_t s,
+                          bool early, A&&... a) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -42,18 +44,21 @@ cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
-  cfg.numAttrs = p.overlap ? 1 : 0;
+  cfg.numAttrs = p.overlap && early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(a)...);
 }
 
-// The fix-up after a fused step kernel (k_fixup); nothing when no node needs it.
+// The fix-up after a fused step kernel (k_fixup); nothing when no node needs it.  `early`: it may start
+// while the step kernel drains.  Not after the persistent pipelines, beside whose CTAs a block of it fits
+// and then holds on to its SM: 100 x 90 x 110 FP16 cavity 35 us a step with a plain launch, 45 with an early one
+// (64^3 21 / 36, 128^3 64 / 86).
 template <typename S, typename R, bool STRICT, bool WALLS>
-cudaError_t launch_fixup(const S* fi, S* fo, const int8_t* flags, const StepPlan& p, bool list, cudaStream_t s) {
+cudaError_t launch_fixup(const S* fi, S* fo, const int8_t* flags, const StepPlan& p, bool list, bool early, cudaStream_t s) {
   const FixGeometry g = fix_geometry(p, list);
   if (g.total == 0) return cudaSuccess;
   const dim3 grid((g.total + FIX_THREADS - 1) / FIX_THREADS);
-  if (p.collision == 0) return launch_kernel(k_fixup<S, R, STRICT, WALLS, 0>, grid, dim3(FIX_THREADS), 0, p, s, fi, fo, flags, p, g);
-  return launch_kernel(k_fixup<S, R, STRICT, WALLS, 1>, grid, dim3(FIX_THREADS), 0, p, s, fi, fo, flags, p, g);
+  if (p.collision == 0) return launch_kernel(k_fixup<S, R, STRICT, WALLS, 0>, grid, dim3(FIX_THREADS), 0, p, s, early, fi, fo, flags, p, g);
+  return launch_kernel(k_fixup<S, R, STRICT, WALLS, 1>, grid, dim3(FIX_THREADS), 0, p, s, early, fi, fo, flags, p, g);
 }
 
 // The face pass after a step kernel that left the boundary operators out: the nodes of the faces
@@ -70,7 +75,7 @@ cudaError_t launch_faces(const S* fi, S* fo, const int8_t* flags, const StepPlan
     }
   if ((faces & 3) == 3 && 2 * int64_t(p.ny) * p.nz > area) area = 2 * int64_t(p.ny) * p.nz;  // x faces interleaved
   const dim3 fgrid(unsigned((area + 255) / 256), 6, 1);
-  if constexpr (MODE == MODE_FUSED) return launch_fixup<S, R, STRICT, WALLS>(fi, fo, flags, p, false, s);
+  if constexpr (MODE == MODE_FUSED) return launch_fixup<S, R, STRICT, WALLS>(fi, fo, flags, p, false, true, s);
   k_faces<S, R, STRICT, MODE, WALLS, 2><<<fgrid, 256, 0, s>>>(fi, fo, flags, p, faces);
   return cudaGetLastError();
 }
@@ -88,9 +93,9 @@ cudaError_t launch_one(const void* fin, void* fout, const int8_t* flags, const S
       constexpr bool FUSED = MODE == MODE_FUSED;
       cudaError_t e;
       if (FUSED && p.collision == 0)
-        e = launch_kernel(k_step_pairs<S, R, STRICT, MODE, WALLS, FUSED ? 0 : 2, MINB>, pgrid, dim3(256), 0, p, s, fi, fo, flags, p);
+        e = launch_kernel(k_step_pairs<S, R, STRICT, MODE, WALLS, FUSED ? 0 : 2, MINB>, pgrid, dim3(256), 0, p, s, true, fi, fo, flags, p);
       else
-        e = launch_kernel(k_step_pairs<S, R, STRICT, MODE, WALLS, FUSED ? 1 : 2, MINB>, pgrid, dim3(256), 0, p, s, fi, fo, flags, p);
+        e = launch_kernel(k_step_pairs<S, R, STRICT, MODE, WALLS, FUSED ? 1 : 2, MINB>, pgrid, dim3(256), 0, p, s, true, fi, fo, flags, p);
       if (e) return e;
       return launch_faces<S, R, STRICT, MODE, WALLS>(fi, fo, flags, p, s);
     }
@@ -98,9 +103,9 @@ cudaError_t launch_one(const void* fin, void* fout, const int8_t* flags, const S
   constexpr bool FUSED = MODE == MODE_FUSED;
   cudaError_t e;
   if (FUSED && p.collision == 0)
-    e = launch_kernel(k_step<S, R, STRICT, MODE, WALLS, FUSED ? 0 : 2, MINB>, grid, block, 0, p, s, fi, fo, flags, p);
+    e = launch_kernel(k_step<S, R, STRICT, MODE, WALLS, FUSED ? 0 : 2, MINB>, grid, block, 0, p, s, true, fi, fo, flags, p);
   else
-    e = launch_kernel(k_step<S, R, STRICT, MODE, WALLS, FUSED ? 1 : 2, MINB>, grid, block, 0, p, s, fi, fo, flags, p);
+    e = launch_kernel(k_step<S, R, STRICT, MODE, WALLS, FUSED ? 1 : 2, MINB>, grid, block, 0, p, s, true, fi, fo, flags, p);
   if (e) return e;
   if constexpr (face_pass_tier<S>()) return launch_faces<S, R, STRICT, MODE, WALLS>(fi, fo, flags, p, s);
   return cudaSuccess;
@@ -135,13 +140,13 @@ cudaError_t launch_vec(int walls, const void* fin, void* fout, const int8_t* fla
   constexpr bool FUSED = MODE == MODE_FUSED;
   cudaError_t e;
   if (FUSED && p.collision == 0)
-    e = launch_kernel(k_step_vec<S, R, STRICT, MODE, NPT, FUSED ? 0 : 2, MINB>, grid, block, 0, p, s, pl, flags, p);
+    e = launch_kernel(k_step_vec<S, R, STRICT, MODE, NPT, FUSED ? 0 : 2, MINB>, grid, block, 0, p, s, true, pl, flags, p);
   else
-    e = launch_kernel(k_step_vec<S, R, STRICT, MODE, NPT, FUSED ? 1 : 2, MINB>, grid, block, 0, p, s, pl, flags, p);
+    e = launch_kernel(k_step_vec<S, R, STRICT, MODE, NPT, FUSED ? 1 : 2, MINB>, grid, block, 0, p, s, true, pl, flags, p);
   if (e || MODE == MODE_PROLOGUE) return e;
   if constexpr (FUSED)
-    return walls ? launch_fixup<S, R, STRICT, true>(fi, fo, flags, p, true, s)
-                 : launch_fixup<S, R, STRICT, false>(fi, fo, flags, p, false, s);
+    return walls ? launch_fixup<S, R, STRICT, true>(fi, fo, flags, p, true, true, s)
+                 : launch_fixup<S, R, STRICT, false>(fi, fo, flags, p, false, true, s);
   if ((e = launch_faces<S, R, STRICT, MODE, false>(fi, fo, flags, p, s))) return e;
   if (!walls) return cudaSuccess;
   k_wall_fixup<S, R, STRICT, MODE, 2><<<unsigned((p.ncell + 255) / 256), 256, 0, s>>>(fi, fo, flags, p);
@@ -268,7 +273,7 @@ cudaError_t launch_rows_t(const Planes<S>& pl, const int8_t* flags, const StepPl
   const size_t smem = rows_smem_bytes(STAGES, g);
   if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return e;
   const int grid = g.ntiles < a.sms * MINB ? g.ntiles : a.sms * MINB;
-  return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, pl, flags, p, g, a.err, a.wait_limit);
+  return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, true, pl, flags, p, g, a.err, a.wait_limit);
 }
 
 template <typename S, int COLL>
@@ -299,7 +304,7 @@ cudaError_t launch_spans_t(const Planes<S>& pl, const int8_t* flags, const StepP
   const size_t smem = spans_smem_bytes(STAGES, g);
   if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return e;
   const int grid = g.ntiles < a.sms * MINB ? g.ntiles : a.sms * MINB;
-  return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, pl, flags, p, g, a.err, a.wait_limit);
+  return launch_kernel(kern, dim3(grid), dim3(32 * (WARPS + 1)), smem, p, s, true, pl, flags, p, g, a.err, a.wait_limit);
 }
 
 // Which pipeline a fused step of `variant` (8 or 9) runs on the lattice: 1 the row pipeline (rows
@@ -333,8 +338,8 @@ cudaError_t launch_rows(int mode, int walls, const void* fin, void* fout, const 
         e = p.collision == 0 ? launch_spans_t<S, 0, 9>(pl, flags, p, g, a, s) : launch_spans_t<S, 1, 9>(pl, flags, p, g, a, s);
     }
     if (e) return e;
-    return walls ? launch_fixup<S, R, STRICT, true>(fi, fo, flags, p, true, s)
-                 : launch_fixup<S, R, STRICT, false>(fi, fo, flags, p, false, s);
+    return walls ? launch_fixup<S, R, STRICT, true>(fi, fo, flags, p, true, false, s)
+                 : launch_fixup<S, R, STRICT, false>(fi, fo, flags, p, false, false, s);
   }
 }
 

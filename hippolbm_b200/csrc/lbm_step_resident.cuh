@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
     uint32_t* dst = reinterpret_cast<uint32_t*>(&p);
     for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += blockDim.x) dst[w] = src[w];
     __syncthreads();
-    const bool pairs = is_16bit<S>() && p.nsets == 0 && !p.has_force && (!p.wall_flags || p.walls);
+    const bool pairs = is_16bit<S>() && p.nsets == 0 && (!p.wall_flags || p.walls);
     if (threadIdx.x == 0) {
       resident_geometry(p, pairs, is_16bit<S>() && !pairs, g);
       p.seed = seed >= 0 ? uint32_t(seed) : L.step[parity];
