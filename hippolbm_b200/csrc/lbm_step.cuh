@@ -1034,7 +1034,7 @@ __device__ __forceinline__ void pair_update(float2 (&v)[Q], const StepPlan& p, i
     Unroll<0, Q>::run([&]<int I>() { v[I] = Lanes<float2>::select(wall, Lanes<float2>::splat(wall_value<S, I>(p)), v[I]); });
 }
 
-template <typename S, bool WALLS, bool LIVE>
+template <typename S, bool WALLS, bool LIVE, bool INNER>
 __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls);
@@ -1048,23 +1048,24 @@ __device__ __forceinline__ void node_gather(const S* __restrict__ fin, const int
   if constexpr (MODE == MODE_PROLOGUE) {
     Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_stream(fin + I * p.stride + idx); });
   } else {
-    node_pull<S, WALLS, false>(fin, flags, p, x, y, z, idx, raw, true);
+    node_pull<S, WALLS, false, true>(fin, flags, p, x, y, z, idx, raw, true);
   }
 }
 
 // node_gather's pull: source coordinates x - e for e in {+1, 0, -1}; periodic axes wrap, others
 // flag "outside" (on-node bounce-back), as do wall sources where wall_bounce_back is active (WALLS
-// and, in kernels that take several plans, `walls`).
-template <typename S, bool WALLS, bool LIVE>
+// and, in kernels that take several plans, `walls`).  INNER: a warp of inner nodes takes a shorter way.
+template <typename S, bool WALLS, bool LIVE, bool INNER>
 __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls) {
-  if constexpr (!LIVE && sizeof(S) < 8) {
+  if constexpr (INNER && !LIVE && sizeof(S) < 8) {
     // A warp of inner nodes needs one constant offset per direction: about 250 instructions of index
     // arithmetic less a node (the one-node FP32 step of a 181 x 150 x 170 channel is bound by issue).
     // Decided per warp: lanes that went different ways would wait for each other's loads.  Measured (us a
     // step): FP32 sphere 150 x 120 x 131 95 -> 84, Poiseuille 130 x 97 x 113 54 -> 51; FP64, bound by bytes,
-    // keeps the one path (sphere 124 -> 132 with two).
+    // keeps the one path (sphere 124 -> 132 with two).  So do the fix-up of a lattice without walls and the span
+    // pipeline, which pull face nodes alone (FP16 channel 181 x 150 x 170: 113 us a step with two, 108 with one).
     const bool inner = x > 0 && x < p.nx - 1 && y > 0 && y < p.ny - 1 && z > 0 && z < p.nz - 1;
     if (__all_sync(__activemask(), inner)) {
       const S* at = fin + idx;
@@ -1350,7 +1351,7 @@ __global__ void __launch_bounds__(FIX_THREADS)
     const int8_t flag = flags[idx];
     const bool walls = near || !g.list;
     S raw[Q];
-    node_pull<S, WALLS, false>(fin, flags, p, x, y, z, idx, raw, walls);
+    node_pull<S, WALLS, false, WALLS>(fin, flags, p, x, y, z, idx, raw, walls);
     Unroll<0, Q>::run([&]<int I>() { v[I] = load_value<S, R, I>(raw[I], p); });
     node_update<S, R, STRICT, MODE_FUSED, COLL>(v, fin, idx, x, y, z, flag, p, true, on_op_face(p, x, y, z));
     if (WALLS && walls && flag == FLAG_WALL) live = false;

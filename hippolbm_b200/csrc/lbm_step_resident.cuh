@@ -150,7 +150,7 @@ __device__ __forceinline__ void resident_face(const S* fin, const int8_t* __rest
   }
   it.idx = (uint32_t(it.z) * uint32_t(p.ny) + uint32_t(it.y)) * uint32_t(p.nx) + uint32_t(it.x);
   it.flag = flags[it.idx];
-  node_pull<S, WALLS, true>(fin, flags, p, it.x, it.y, it.z, it.idx, raw, walls);
+  node_pull<S, WALLS, true, false>(fin, flags, p, it.x, it.y, it.z, it.idx, raw, walls);
 }
 
 // The update and store of a fetched node (a wall node keeps its scratch).
@@ -210,11 +210,11 @@ __device__ __forceinline__ void resident_pair(const S* fin, S* fout, const int8_
       const unsigned short near = __ldg(reinterpret_cast<const unsigned short*>(p.nearwall + n));
       S raw[Q];
       if (a && (near & 0xff) == 1) {
-        node_pull<S, true, true>(fin, flags, p, x, y, z, n, raw, true);
+        node_pull<S, true, true, false>(fin, flags, p, x, y, z, n, raw, true);
         Unroll<0, Q>::run([&]<int I>() { w[I] = (w[I] & 0xffff0000u) | uint32_t(PackedChunk<S, 2>::bits(raw[I])); });
       }
       if (b && (near >> 8) == 1) {
-        node_pull<S, true, true>(fin, flags, p, x + 1, y, z, n + 1, raw, true);
+        node_pull<S, true, true, false>(fin, flags, p, x + 1, y, z, n + 1, raw, true);
         Unroll<0, Q>::run([&]<int I>() { w[I] = (w[I] & 0xffffu) | uint32_t(PackedChunk<S, 2>::bits(raw[I])) << 16; });
       }
     }
