@@ -480,7 +480,8 @@ int resident_steps(hlbm_ctx* c, int64_t nsteps) {
   a.nbars = 1;
   a.err = c->err_dev;
   a.grid = int(std::min<int64_t>(c->sms, (c->ncell + 63) / 64));
-  a.wait_limit = c->wait_limit;
+  // the caller's bound in the tiers whose default kernels always waited (hlbm_set_wait_limit)
+  a.wait_limit = elem_size(c->precision) == 2 ? c->wait_limit : TMA_WAIT_LIMIT;
   while (nsteps > 0) {
     const int m = int(std::min<int64_t>(nsteps, RESIDENT_STEPS));
     a.one = ResidentTask{0, 0, a.grid, 0, m};

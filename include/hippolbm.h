@@ -198,12 +198,15 @@ int hlbm_info(hlbm_ctx* ctx, int64_t info[8]);
  * 0 = one node per thread (two per thread for the 16-bit tiers), 1 = vectorised (consecutive
  * x-nodes per thread in one vector per direction plane -- 16 bytes at variant 1, 8 bytes at 3 and
  * 5 for the FP32 and 16-bit tiers, 16 bytes always for FP64; used when nx splits into >= 32
- * vectors, else the first kernel runs; with wall obstacles a fix-up pass re-steps the nodes next
+ * vectors, else the first kernel runs; with wall obstacles a fix-up launch re-steps the nodes next
  * to walls); variant / 2 = 0, 1, 2 targets at least 1, 2 or 3 blocks of 256 threads per SM.
- * The FP32 and 16-bit tiers update node pairs in packed FP32 where a plan has no body force, no
- * start_iteration boxes and no wall nodes outside wall_bounce_back; other plans run one node per
- * thread.  A context starts at its tier's default (hlbm_autotune's pick on 512^3 Couette: FP64 4,
- * FP32 1, FP16 / BF16 9) until hlbm_tune or hlbm_autotune chooses.  Variants 6, 7: persistent
+ * The FP32 and 16-bit tiers update node pairs in packed FP32 where a plan has no start_iteration
+ * boxes, no wall nodes outside wall_bounce_back and, with 16-bit MRT, no body force; other plans run
+ * one node per thread.  A context starts at its tier's default (hlbm_autotune's pick on 512^3 Couette:
+ * FP64 4, FP32 1, FP16 / BF16 9; 4 instead of 9 where rows are ragged and some face is no boundary
+ * operator's) until hlbm_tune or hlbm_autotune chooses.  Until hlbm_tune chooses, hlbm_step advances
+ * lattices that fit the GPU at one node per thread, and 16-bit BGK lattices of up to 50 MB, by many steps
+ * a launch (not while the context's stream is being captured).  Variants 6, 7: persistent
  * kernel fed by bulk asynchronous copies of whole rows
  * into shared-memory stages (256 or 512 threads per CTA; needs nx * bytes per population to be a
  * multiple of 16; otherwise variant 4 runs).  hlbm_autotune times `reps` fused launches of every
@@ -212,9 +215,9 @@ int hlbm_info(hlbm_ctx* ctx, int64_t info[8]);
  * skipped) in ms_per_variant[HLBM_NUM_VARIANTS].  Variants 8, 9 (FP16 / BF16): the row pipeline --
  * a producer warp bulk-copies each tile's source rows and flags into shared-memory stages,
  * consumer warps update node pairs from there in packed FP32 -- with two CTAs of 8 consumer warps
- * (8) or one CTA of 12 (9) per SM; fused steps of lattices with nx % 16 == 0, nx <= 1024 (8) or
- * 1536 (9) and the pair kernels' plan conditions.  Other lattices with nx >= 4, fewer than 2^32
- * nodes and those plan conditions take the span pipeline at the same shape: tiles are spans of
+ * (8) or one CTA of 12 or, where rows fill it better, 15 (9) per SM; fused steps of lattices with
+ * nx % 16 == 0, nx <= 1024 (8) or 1536 (9) and the pair kernels' plan conditions.  Other lattices
+ * with nx >= 4, fewer than 2^32 nodes and those plan conditions take the span pipeline at the same shape: tiles are spans of
  * the linear node index, one bulk copy per direction, so rows of any length stream from shared
  * memory.  Otherwise variant 5 runs. */
 #define HLBM_NUM_VARIANTS 10
@@ -222,9 +225,9 @@ int hlbm_tune(hlbm_ctx* ctx, int32_t variant);
 int hlbm_autotune(hlbm_ctx* ctx, int32_t reps, int32_t* chosen, double* ms_per_variant);
 /* the context's cudaStream_t, as a pointer-sized handle */
 void* hlbm_stream(hlbm_ctx* ctx);
-/* Bound on each wait of the pipelined kernels (variants 6 - 9) in polls of their shared-memory
- * barriers (the first poll a test, the others a hardware-suspended try_wait of up to about a
- * microsecond); 0 restores the default of 2e7 polls.  Every wait also gives up after two seconds
+/* Bound on each wait of the pipelined kernels (variants 6 - 9) and of the many-step launches of the
+ * 16-bit tiers in polls of their barriers (in shared memory the first poll is a test, the others a hardware-suspended try_wait
+ * of up to about a microsecond); 0 restores the default of 2e7 polls.  Every wait also gives up after two seconds
  * whatever the bound.  No reference counterpart.  A wait that runs
  * out records an error on the device and its CTA returns after its copies in flight have landed;
  * the next call that reads the state (hlbm_get_populations, hlbm_simulation_state, ...) fails with
