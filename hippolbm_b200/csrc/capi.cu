@@ -20,6 +20,7 @@
 
 #include "aux_kernels.cuh"
 #include "hippolbm.h"
+#include "host_copy.h"
 #include "launch.cuh"
 #include "lbm_step_resident.cuh"
 #include "observe.cuh"
@@ -98,6 +99,8 @@ cudaError_t pool_alloc(void** ptr, size_t bytes, int dev, cudaStream_t s) {
   if (!pool) return cudaErrorMemoryAllocation;
   return cudaMallocFromPoolAsync(ptr, bytes, pool, s);
 }
+
+HostCopy g_host_copy;
 
 void pool_free(void* ptr, cudaStream_t s) {
   if (ptr) cudaFreeAsync(ptr, s);
@@ -1048,8 +1051,8 @@ int hlbm_macro_variables(hlbm_ctx* c, double* rho, double* u) {
   base_plan(c, p);
   c->launches += 2;
   cudaError_t e = launch_macro_stats(c->precision, s, c->flags, p, drho, du, c->partials, c->stats_dev, c->stream);
-  if (e == cudaSuccess && rho) e = cudaMemcpyAsync(rho, drho, n * 8, cudaMemcpyDeviceToHost, c->stream);
-  if (e == cudaSuccess && u) e = cudaMemcpyAsync(u, du, 3 * n * 8, cudaMemcpyDeviceToHost, c->stream);
+  if (e == cudaSuccess && rho) e = g_host_copy.copy(rho, drho, n * 8, c->stream);
+  if (e == cudaSuccess && u) e = g_host_copy.copy(u, du, 3 * n * 8, c->stream);
   pool_free(drho, c->stream);
   pool_free(du, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1145,17 +1148,32 @@ int hlbm_get_populations(hlbm_ctx* c, double* out) {
   if (int rc = state_buffer(c, &s)) return rc;
   const size_t n = size_t(c->ncell);
   if (elem_size(c->precision) == 8) {
-    HLBM_CK(cudaMemcpy2DAsync(out, n * 8, s, size_t(c->stride) * 8, n * 8, Q, cudaMemcpyDeviceToHost, c->stream));
+    HLBM_CK(g_host_copy.copy_rows(out, s, size_t(c->stride) * 8, n * 8, Q, c->stream));
   } else {
-    if (!c->plane_tmp && pool_alloc((void**)&c->plane_tmp, n * 8, c->device, c->stream) != cudaSuccess)
-      return fail(HLBM_ENOMEM, "hlbm_get_populations: no memory");
+    // several directions at a time, decoded side by side: about 64 MB, at least one; one where memory is short
+    size_t group = std::min<size_t>(Q, std::max<size_t>(1, (size_t(64) << 20) / (n * 8)));
+    double* tmp = nullptr;
+    if (pool_alloc((void**)&tmp, group * n * 8, c->device, c->stream) != cudaSuccess) {
+      cudaGetLastError();
+      group = 1;
+      if (pool_alloc((void**)&tmp, n * 8, c->device, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(HLBM_ENOMEM, "hlbm_get_populations: no memory");
+      }
+    }
     StepPlan p;
     base_plan(c, p);
-    for (int i = 0; i < Q; i++) {
-      c->launches++;
-      HLBM_CK(launch_decode(c->precision, s, c->plane_tmp, i, p, c->stream));
-      HLBM_CK(cudaMemcpyAsync(out + i * n, c->plane_tmp, n * 8, cudaMemcpyDeviceToHost, c->stream));
+    cudaError_t e = cudaSuccess;
+    for (size_t i = 0; i < size_t(Q) && e == cudaSuccess; i += group) {
+      const size_t k = std::min(group, size_t(Q) - i);
+      for (size_t j = 0; j < k && e == cudaSuccess; j++) {
+        c->launches++;
+        e = launch_decode(c->precision, s, tmp + j * n, int(i + j), p, c->stream);
+      }
+      if (e == cudaSuccess) e = g_host_copy.copy(out + i * n, tmp, k * n * 8, c->stream);
     }
+    pool_free(tmp, c->stream);
+    if (e != cudaSuccess) return fail(HLBM_ECUDA, std::string("hlbm_get_populations: ") + cudaGetErrorString(e));
   }
   HLBM_CK(cudaStreamSynchronize(c->stream));
   return HLBM_OK;
@@ -1923,6 +1941,7 @@ void* hlbm_batch_stream(hlbm_batch* b) { return b ? (void*)b->stream : nullptr; 
 
 int hlbm_trim_memory(int32_t device) {
   if (device < 0 || device >= 64) return fail(HLBM_EINVAL, "hlbm_trim_memory: bad device");
+  g_host_copy.release();
   cudaMemPool_t pool = nullptr;
   {
     std::lock_guard<std::mutex> lock(g_pool_mutex);

@@ -78,7 +78,8 @@ int hlbm_destroy(hlbm_ctx* ctx);
 /* Device memory of contexts and batches comes from a stream-ordered pool per device that keeps
  * freed blocks for the next allocation, so that creating and destroying lattices while others run
  * costs no device-wide synchronisation (no reference counterpart).  hlbm_trim_memory waits for the
- * device and returns the pool's unused blocks to the driver. */
+ * device and returns the pool's unused blocks to the driver, and gives back the 16 MiB of pinned
+ * memory that read-outs of 4 MB and more into pageable arrays share. */
 int hlbm_trim_memory(int32_t device);
 
 /* lbm_parameters (lbm_parameters.cpp:73-99): tau if has_tau, else dt if dt > 0, else the
@@ -226,8 +227,8 @@ int hlbm_autotune(hlbm_ctx* ctx, int32_t reps, int32_t* chosen, double* ms_per_v
 /* the context's cudaStream_t, as a pointer-sized handle */
 void* hlbm_stream(hlbm_ctx* ctx);
 /* Bound on each wait of the pipelined kernels (variants 6 - 9) and of the many-step launches of the
- * 16-bit tiers in polls of their barriers (in shared memory the first poll is a test, the others a hardware-suspended try_wait
- * of up to about a microsecond); 0 restores the default of 2e7 polls.  Every wait also gives up after two seconds
+ * 16-bit tiers in polls of their barriers (in shared memory the first poll is a test, the others a
+ * hardware-suspended try_wait of up to about a microsecond); 0 restores the default of 2e7 polls.  Every wait also gives up after two seconds
  * whatever the bound.  No reference counterpart.  A wait that runs
  * out records an error on the device and its CTA returns after its copies in flight have landed;
  * the next call that reads the state (hlbm_get_populations, hlbm_simulation_state, ...) fails with
