@@ -223,10 +223,12 @@ __device__ __forceinline__ void rows_read_interior(const S* row, int x0, uint32_
   }
 }
 
+// The plan is a plain parameter: as a __grid_constant__ one the kernel came out 7 % slower (FP16 Couette 512^3
+// 1748 us a step against 1629, 256^3 238 / 223, 320^3 MRT 546 / 542).
 template <typename S, int COLL, int STAGES, int WARPS, int MINB>
 __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
-    k_step_rows(const __grid_constant__ Planes<S> pl, const int8_t* __restrict__ flags, const __grid_constant__ StepPlan p,
-                const __grid_constant__ RowsGeometry g, int* __restrict__ err, long long wait_limit) {
+    k_step_rows(const __grid_constant__ Planes<S> pl, const int8_t* __restrict__ flags, const StepPlan p,
+                RowsGeometry g, int* __restrict__ err, long long wait_limit) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw);
   uint64_t* empty = full + STAGES;
