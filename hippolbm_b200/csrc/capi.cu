@@ -250,7 +250,6 @@ void base_plan(hlbm_ctx* c, StepPlan& p) {
     p.pull[i] = i * p.stride - ((int64_t(D3Q19::ez[i]) * p.ny + D3Q19::ey[i]) * p.nx + D3Q19::ex[i]);
   p.rho0 = c->rho0;
   p.nearwall = c->nearwall;
-  p.overlap = 1;
   p.wall_flags = c->maybe_walls ? 1 : 0;
   p.scale = c->scale;
   p.inv_scale = 1.0 / c->scale;
@@ -1006,11 +1005,10 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
   if (nsteps == 0) return HLBM_OK;
   if (int rc = set_device(c)) return rc;
   if (int rc = build_plan(c)) return rc;
-  // a caller's graph holds one plain launch a step: no cooperative launch, no overlapped ones
+  // a caller's graph holds plain launches: no cooperative one, no overlapped ones
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   HLBM_CK(cudaStreamIsCapturing(c->stream, &capture));
   const bool captured = capture != cudaStreamCaptureStatusNone;
-  c->plan.overlap = !captured;
   if (c->phase == MATER) c->phase = POSTCOL;
   if (c->phase == RAW) {
     HLBM_CK(launch_step_kernel(c, MODE_PROLOGUE, c->f[c->cur], c->f[1 - c->cur]));
@@ -1020,8 +1018,13 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
     nsteps--;
   }
   if (nsteps > 0 && !captured && resident_applies(c)) return resident_steps(c, nsteps);
+  // The call's first step is launched plainly, and the ones after it may overlap the kernel before them: that is
+  // then one of this call's own, which write populations only (pdl_begin).
   for (int64_t s = 0; s < nsteps; s++) {
-    HLBM_CK(launch_step_kernel(c, MODE_FUSED, c->f[c->cur], c->f[1 - c->cur]));
+    const cudaError_t e = launch_step_kernel(c, MODE_FUSED, c->f[c->cur], c->f[1 - c->cur]);
+    c->plan.overlap = 0;
+    HLBM_CK(e);
+    c->plan.overlap = !captured && s + 1 < nsteps;
     c->cur = 1 - c->cur;
     c->steps++;
   }
@@ -1489,7 +1492,6 @@ int batch_capture_concurrent(hlbm_batch* b) {
       StepPlan pk = c->plan;
       pk.seed_dev = sr ? c->seed_dev : nullptr;
       pk.seed_parity = k;
-      pk.overlap = 0;
       e = launch_with_plan(c, MODE_FUSED, c->f[c->cur ^ k], c->f[c->cur ^ k ^ 1], pk, concurrent_variant(c), c->stream);
     }
     if (e == cudaSuccess) e = cudaEventRecord(c->join_ev, c->stream);
@@ -1883,10 +1885,9 @@ int hlbm_batch_autotune(hlbm_batch* b, int32_t reps, int32_t* chosen, double* ms
         if (e == cudaSuccess && !c->join_ev) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, b->fork_ev, 0);
         StepPlan pk = c->plan;
-        pk.overlap = 0;
-        if (e == cudaSuccess)
+          if (e == cudaSuccess)
           e = launch_with_plan(c, c->phase == RAW ? MODE_PROLOGUE : MODE_FUSED, c->f[c->cur], c->f[1 - c->cur],
-                               pk, concurrent_variant(c), c->stream);
+                               c->plan, concurrent_variant(c), c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(c->join_ev, c->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, c->join_ev, 0);
       }

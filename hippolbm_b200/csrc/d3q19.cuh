@@ -77,7 +77,7 @@ struct StepPlan {
   // when set, the step number comes from seed_dev[seed_parity] instead of `seed`, and the launch
   // writes seed_dev[seed_parity ^ 1] = that + 1 (launches replayed from a captured graph)
   uint32_t* seed_dev;
-  int32_t overlap;  // step launches may start while the launch before them drains (never in captured graphs)
+  int32_t overlap;  // this launch may start while the step launch before it drains (lbm_step.cuh: pdl_begin)
   int32_t seed_parity;
   // geometry of the one-node-per-thread kernel: 0 = x on threadIdx.x, y on threadIdx.y (rows of
   // whole warps); 1 = blocks of 256 consecutive nodes of a z-plane, for rows that would leave

@@ -31,7 +31,7 @@ inline void step_geometry(const StepPlan& p, dim3& grid, dim3& block) {
 }
 
 // A launch on stream s; with p.overlap and `early` it may start while the launch before it drains
-// (pdl_wait).
+// (pdl_begin).
 template <class... P, class... A>
 cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, const StepPlan& p, cudaStream_t s,
                           bool early, A&&... a) {

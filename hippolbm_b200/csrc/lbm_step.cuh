@@ -30,14 +30,16 @@
 
 namespace hlbm {
 
-// Programmatic dependent launches (StepPlan::overlap).  pdl_wait returns when every launch before this
-// one has finished and its stores are visible; at once for a launch without the attribute.
-// pdl_begin opens a step kernel: after the wait the next launch of the stream may be scheduled,
-// while this one runs -- it sets up, and the fix-up even reads fin, which is complete by then, before
-// its own wait.  That takes the launch gap (about 2 us) and cold instruction fetches off the step.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Programmatic dependent launches (StepPlan::overlap): a launch may be scheduled while the one before it
+// drains, which takes the launch gap (about 2 us) off the step.  pdl_begin stands before a kernel's first
+// read or write of memory: it returns when every launch before this one has finished and its stores are
+// visible (at once for a launch without the attribute), and only then lets the next launch be scheduled.
+// So of several queued launches at most one has passed its wait at a time; the others only set up.
+// What the launch before may still be writing while this one waits are the populations, so they are
+// read by coherent loads behind the wait (ld_pop); flags, maps and lists may take the read-only path,
+// because the first launch of an hlbm_step call is a plain one and nothing after it writes them.
 __device__ __forceinline__ void pdl_begin() {
-  pdl_wait();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
@@ -149,18 +151,38 @@ struct Codec<__nv_bfloat16, float> {
   }
 };
 
-template <typename S>
-__device__ __forceinline__ S ld_stream(const S* p) {
-  return __ldg(p);
+// A population read (V: a value or an aligned vector of them) by an ordinary, coherent load, which stays
+// behind the wait that opens an overlapped launch (pdl_begin).  The read-only path (__ldg, or a
+// const __restrict__ pointer) is defined only for data that nobody writes while the kernel lives, so
+// population pointers carry no __restrict__.
+template <typename V>
+__device__ __forceinline__ V ld_stream(const V* p) {
+  return *p;
 }
-// A population read. LIVE: the lattice is written by other SMs inside this launch (the resident
-// kernel), so the read goes to L2.
-template <bool LIVE, typename S>
-__device__ __forceinline__ S ld_pop(const S* p) {
-  if constexpr (LIVE)
-    return __ldcg(p);
-  else
+// LIVE: the lattice is written by other SMs inside this launch (the resident kernel), so the read goes past
+// L1, and volatile keeps it behind the group barrier.
+template <bool LIVE, typename V>
+__device__ __forceinline__ V ld_pop(const V* p) {
+  if constexpr (!LIVE) {
     return ld_stream(p);
+  } else {
+    static_assert(sizeof(V) == 2 || sizeof(V) == 4 || sizeof(V) == 8, "a population or a word of two");
+    V v;
+    if constexpr (sizeof(V) == 2) {
+      unsigned short b;
+      asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(b) : "l"(p));
+      memcpy(&v, &b, 2);
+    } else if constexpr (sizeof(V) == 4) {
+      uint32_t b;
+      asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(b) : "l"(p));
+      memcpy(&v, &b, 4);
+    } else {
+      uint64_t b;
+      asm volatile("ld.global.cg.u64 %0, [%1];" : "=l"(b) : "l"(p));
+      memcpy(&v, &b, 8);
+    }
+    return v;
+  }
 }
 
 // ------------------------------------------------------------------ storage rounding
@@ -774,7 +796,7 @@ __device__ __forceinline__ bool on_face(int x, int y, int z, const StepPlan& p) 
 // (post_bounce_back.cu:115-120): the value saved by pre_bounce_back is this node's own
 // post-collision opposite population, plus the cavity increments of that face.
 template <typename S, typename R, bool LIVE>
-__device__ __forceinline__ void post_bb(R (&v)[Q], const S* __restrict__ fin, int64_t idx, int x, int y, int z,
+__device__ __forceinline__ void post_bb(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z,
                                         const StepPlan& p) {
   Unroll<0, 6>::run([&]<int F>() {
     if (p.periodic[F / 2]) return;
@@ -806,7 +828,7 @@ __device__ __forceinline__ void cavity_increments(R (&v)[Q], int z, const StepPl
 // the upstream node, or the node's own opposite one where the upstream node is outside a
 // non-periodic face or (wall_bounce_back active) a wall.
 template <typename S, typename R, int I>
-__device__ __forceinline__ R pull_value(const S* __restrict__ fin, const int8_t* __restrict__ flags,
+__device__ __forceinline__ R pull_value(const S* fin, const int8_t* __restrict__ flags,
                                         const StepPlan& p, int x, int y, int z) {
   constexpr int O = D3Q19::opp(I);
   int sx = x - D3Q19::ex[I], sy = y - D3Q19::ey[I], sz = z - D3Q19::ez[I];
@@ -830,7 +852,7 @@ __device__ __forceinline__ R pull_value(const S* __restrict__ fin, const int8_t*
 // outlet code.  It reads only entering slots and interior nodes' slots, never the slots it
 // writes.  (a, b) are the node's coordinates along the face's two other axes, in x, y, z order.
 template <typename S, typename R, int F>
-__device__ __forceinline__ void zero_gradient_node(S* __restrict__ fin, const int8_t* __restrict__ flags,
+__device__ __forceinline__ void zero_gradient_node(S* fin, const int8_t* __restrict__ flags,
                                                    const StepPlan& p, int a, int b) {
   constexpr int axis = F / 2;
   const int c = (F & 1) ? (axis == 0 ? p.nx : (axis == 1 ? p.ny : p.nz)) - 1 : 0;
@@ -848,7 +870,7 @@ __device__ __forceinline__ void zero_gradient_node(S* __restrict__ fin, const in
 }
 
 template <typename S, typename R, bool LIVE>
-__device__ __forceinline__ void plane_ops(R (&v)[Q], const S* __restrict__ fin, int64_t idx, int x, int y, int z,
+__device__ __forceinline__ void plane_ops(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z,
                                           int8_t flag, const StepPlan& p) {
   for (int o = 0; o < p.nops; o++) {
     const PlaneOp& op = p.ops[o];
@@ -1000,7 +1022,7 @@ __device__ __forceinline__ bool on_op_z_face(const StepPlan& p, int z) {
 // collision.  The 16-bit tiers carry scaled deviations; the boundary operators and the boxes work
 // on full populations, so those nodes convert around them.
 template <typename S, typename R, bool STRICT, int MODE, int COLL, bool LIVE = false>
-__device__ __forceinline__ void node_update(R (&v)[Q], const S* __restrict__ fin, int64_t idx, int x, int y, int z,
+__device__ __forceinline__ void node_update(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z,
                                             int8_t flag, const StepPlan& p, bool pulled, bool edge) {
   constexpr bool DEV = is_16bit<S>();
   if (pulled && edge && p.nops > 0) {
@@ -1035,7 +1057,7 @@ __device__ __forceinline__ void pair_update(float2 (&v)[Q], const StepPlan& p, i
 }
 
 template <typename S, bool WALLS, bool LIVE, bool INNER>
-__device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
+__device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls);
 
@@ -1043,7 +1065,7 @@ __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_
 // in the prologue its own values), every load issued before any is used.  A bounced value (the
 // node's own opp(I) slot) decodes like a pulled one because the storage reference is symmetric.
 template <typename S, int MODE, bool WALLS>
-__device__ __forceinline__ void node_gather(const S* __restrict__ fin, const int8_t* __restrict__ flags,
+__device__ __forceinline__ void node_gather(const S* fin, const int8_t* __restrict__ flags,
                                             const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q]) {
   if constexpr (MODE == MODE_PROLOGUE) {
     Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_stream(fin + I * p.stride + idx); });
@@ -1056,7 +1078,7 @@ __device__ __forceinline__ void node_gather(const S* __restrict__ fin, const int
 // flag "outside" (on-node bounce-back), as do wall sources where wall_bounce_back is active (WALLS
 // and, in kernels that take several plans, `walls`).  INNER: a warp of inner nodes takes a shorter way.
 template <typename S, bool WALLS, bool LIVE, bool INNER>
-__device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_t* __restrict__ flags,
+__device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls) {
   if constexpr (INNER && !LIVE && sizeof(S) < 8) {
@@ -1123,7 +1145,7 @@ __device__ __forceinline__ void node_pull(const S* __restrict__ fin, const int8_
 // The whole step for the node (x, y, z): gather, boundary operators (unless OPS is false: a face
 // pass applies them), start_iteration boxes, collision, store.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL, bool OPS = true>
-__device__ __forceinline__ void node_step(const S* __restrict__ fin, S* __restrict__ fout,
+__device__ __forceinline__ void node_step(const S* fin, S* __restrict__ fout,
                                           const int8_t* __restrict__ flags, const StepPlan& p, int x, int y, int z) {
   const int64_t idx = ((int64_t)z * p.ny + y) * p.nx + x;
   const int8_t flag = flags[idx];
@@ -1151,7 +1173,7 @@ constexpr bool face_pass_tier() {
 
 // ------------------------------------------------------------------ the step kernel
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_step(const S* __restrict__ fin, S* __restrict__ fout,
+__global__ void __launch_bounds__(256, MINB) k_step(const S* fin, S* __restrict__ fout,
                                                     const int8_t* __restrict__ flags, const StepPlan p) {
   pdl_begin();
   advance_seed<S, MODE>(p);
@@ -1188,7 +1210,7 @@ __global__ void __launch_bounds__(256, MINB) k_step(const S* __restrict__ fin, S
 // of a wall (population 0); the one-node kernel leaves that slot untouched, and no fluid node
 // reads it either way.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_step_pairs(const S* __restrict__ fin, S* __restrict__ fout,
+__global__ void __launch_bounds__(256, MINB) k_step_pairs(const S* fin, S* __restrict__ fout,
                                                           const int8_t* __restrict__ flags, const StepPlan p) {
   static_assert(is_16bit<S>(), "packed pairs are 16-bit storage");
   pdl_begin();
@@ -1235,7 +1257,7 @@ __global__ void __launch_bounds__(256, MINB) k_step_pairs(const S* __restrict__ 
 // operators.  Both read only fin, so the pass overwrites those nodes' outputs with the complete
 // update.  blockIdx.y is the face; nodes on two faces are computed twice, to the same bits.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL>
-__global__ void __launch_bounds__(256) k_faces(const S* __restrict__ fin, S* __restrict__ fout,
+__global__ void __launch_bounds__(256) k_faces(const S* fin, S* __restrict__ fout,
                                                const int8_t* __restrict__ flags, const StepPlan p, int faces) {
   const int F = blockIdx.y;
   if (!(faces >> F & 1)) return;
@@ -1270,8 +1292,7 @@ __global__ void __launch_bounds__(256) k_faces(const S* __restrict__ fin, S* __r
 
 // The fix-up after a fused step: the nodes on the operator faces, and (list) those next to walls after
 // the kernels that pull without testing for walls, each once and whole by the one-node step.  It
-// reads only fin, as the step kernel does, and overwrites that kernel's results, so it gathers and
-// collides before it waits for it.  One launch, 128 threads a block (more blocks for the few nodes
+// reads only fin, as the step kernel does, and overwrites that kernel's results.  One launch, 128 threads a block (more blocks for the few nodes
 // there are, and one fits beside a pipeline CTA).  The face pass and the scan of the near-wall map that it
 // replaces took 23 + 31 us after a 45 us span kernel on a 150 x 120 x 131 sphere.
 struct FixGeometry {
@@ -1297,9 +1318,9 @@ constexpr int FIX_THREADS = 128;
 
 template <typename S, typename R, bool STRICT, bool WALLS, int COLL>
 __global__ void __launch_bounds__(FIX_THREADS)
-    k_fixup(const S* __restrict__ fin, S* __restrict__ fout, const int8_t* __restrict__ flags,
+    k_fixup(const S* fin, S* __restrict__ fout, const int8_t* __restrict__ flags,
             const __grid_constant__ StepPlan p, const __grid_constant__ FixGeometry g) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_begin();
   uint32_t i = blockIdx.x * FIX_THREADS + threadIdx.x;
   const uint32_t nx = p.nx, ny = p.ny;
   int x = -1, y = 0, z = 0;
@@ -1356,7 +1377,6 @@ __global__ void __launch_bounds__(FIX_THREADS)
     node_update<S, R, STRICT, MODE_FUSED, COLL>(v, fin, idx, x, y, z, flag, p, true, on_op_face(p, x, y, z));
     if (WALLS && walls && flag == FLAG_WALL) live = false;
   }
-  pdl_wait();
   if (live) store_node<S, R, MODE_FUSED>(v, p, launch_seed<S>(p), idx, [&]<int I>(S s) { fout[I * p.stride + idx] = s; });
 }
 
@@ -1365,7 +1385,7 @@ __global__ void __launch_bounds__(FIX_THREADS)
 // step with the wall test, and a read-out gives wall nodes the read-out value of a wall.  It runs
 // after the face pass and reads only fin, so its result replaces both.
 template <typename S, typename R, bool STRICT, int MODE, int COLL>
-__global__ void __launch_bounds__(256) k_wall_fixup(const S* __restrict__ fin, S* __restrict__ fout,
+__global__ void __launch_bounds__(256) k_wall_fixup(const S* fin, S* __restrict__ fout,
                                                     const int8_t* __restrict__ flags, const StepPlan p) {
   const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= p.ncell) return;

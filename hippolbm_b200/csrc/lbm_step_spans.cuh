@@ -116,6 +116,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
   __syncthreads();
 
   if (warp == 0) {  // ------------------------------------------------------------ producer
+    bulk_reads_begin();
     int k = 0;
     for (int t = blockIdx.x; t < g.ntiles; t += gridDim.x, k++) {
       const int s = k % STAGES;

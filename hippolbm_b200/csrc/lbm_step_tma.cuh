@@ -117,6 +117,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, long l
   return false;
 }
 
+// Once, by the threads that issue bulk copies, after pdl_begin: what launches before this one stored by
+// ordinary stores is read by the copies (the asynchronous proxy).
+__device__ __forceinline__ void bulk_reads_begin() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
 // bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned) global -> shared
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile(

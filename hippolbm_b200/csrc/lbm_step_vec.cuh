@@ -29,7 +29,7 @@ template <typename S, int NPT, typename V>
 struct ArrayChunk {
   S e[NPT];
   __device__ __forceinline__ void load(const S* p) {
-    const V v = __ldg(reinterpret_cast<const V*>(p));
+    const V v = ld_stream(reinterpret_cast<const V*>(p));
     static_assert(sizeof(V) == sizeof(S) * NPT, "vector width");
     const S* s = reinterpret_cast<const S*>(&v);
 #pragma unroll
@@ -90,13 +90,13 @@ struct PackedChunk {
   unsigned w[W];
   __device__ __forceinline__ void load(const S* p) {
     if constexpr (W == 4) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+      const uint4 v = ld_stream(reinterpret_cast<const uint4*>(p));
       w[0] = v.x;
       w[1] = v.y;
       w[2] = v.z;
       w[3] = v.w;
     } else {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      const uint2 v = ld_stream(reinterpret_cast<const uint2*>(p));
       w[0] = v.x;
       w[1] = v.y;
     }

@@ -25,7 +25,7 @@ __device__ __forceinline__ double readout_value(R v, const StepPlan& p) {
 
 // out: {sum rho, min |u|, max |u|}; done: blocks finished, zero between launches
 template <typename S, typename R, bool STRICT, bool WALLS>
-__global__ void __launch_bounds__(256) k_observe(const S* __restrict__ fin, const int8_t* __restrict__ flags,
+__global__ void __launch_bounds__(256) k_observe(const S* fin, const int8_t* __restrict__ flags,
                                                  const __grid_constant__ StepPlan p, double* __restrict__ partials,
                                                  unsigned* __restrict__ done, double* __restrict__ out) {
   double s = 0.0, vmin = 1.79769313486231570815e+308, vmax = -1.79769313486231570815e+308;
