@@ -72,45 +72,70 @@ cudaError_t launch_double_couette(int prec, void* f, const StepPlan& p, int dim,
 }
 
 // ------------------------------------------------------------------ zero-gradient outlet pass
-// The pass over one face of lattice m of a descriptor array (lbm_step.cuh: zero_gradient_node),
-// run before each step that pulls from f[cur ^ parity].
+// The pass over one face (lbm_step.cuh: zero_gradient_node), run before each step that pulls from fin.
 template <typename S, typename R>
-__global__ void __launch_bounds__(256) k_zero_gradient(const LatticeDesc* __restrict__ lats, int m, int face,
-                                                       int parity) {
-  __shared__ StepPlan sp;
-  const LatticeDesc L = lats[m];
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(L.plan);
-  uint32_t* dst = reinterpret_cast<uint32_t*>(&sp);
-  for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += blockDim.x) dst[w] = src[w];
-  __syncthreads();
-  const StepPlan& p = sp;
-  S* fin = static_cast<S*>(L.f[L.cur ^ parity]);
+__device__ __forceinline__ void zero_gradient_face(S* fin, const int8_t* __restrict__ flags, const StepPlan& p, int face) {
   const int axis = face / 2;
   const int na = axis == 0 ? p.ny : p.nx, nb = axis == 2 ? p.ny : p.nz;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < int64_t(na) * nb;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int a = int(k % na), b = int(k / na);
     switch (face) {
-      case 0: zero_gradient_node<S, R, 0>(fin, L.flags, p, a, b); break;
-      case 1: zero_gradient_node<S, R, 1>(fin, L.flags, p, a, b); break;
-      case 2: zero_gradient_node<S, R, 2>(fin, L.flags, p, a, b); break;
-      case 3: zero_gradient_node<S, R, 3>(fin, L.flags, p, a, b); break;
-      case 4: zero_gradient_node<S, R, 4>(fin, L.flags, p, a, b); break;
-      default: zero_gradient_node<S, R, 5>(fin, L.flags, p, a, b); break;
+      case 0: zero_gradient_node<S, R, 0>(fin, flags, p, a, b); break;
+      case 1: zero_gradient_node<S, R, 1>(fin, flags, p, a, b); break;
+      case 2: zero_gradient_node<S, R, 2>(fin, flags, p, a, b); break;
+      case 3: zero_gradient_node<S, R, 3>(fin, flags, p, a, b); break;
+      case 4: zero_gradient_node<S, R, 4>(fin, flags, p, a, b); break;
+      default: zero_gradient_node<S, R, 5>(fin, flags, p, a, b); break;
     }
   }
 }
 
+// of a lattice stepped alone, whose plan is the launch's parameter
+template <typename S, typename R>
+__global__ void __launch_bounds__(256) k_zero_gradient(S* fin, const int8_t* __restrict__ flags,
+                                                       const __grid_constant__ StepPlan p, int face) {
+  zero_gradient_face<S, R>(fin, flags, p, face);
+}
+
+// of lattice m of a batch's descriptor array, reading f[cur ^ parity]
+template <typename S, typename R>
+__global__ void __launch_bounds__(256) k_zero_gradient_member(const LatticeDesc* __restrict__ lats, int m, int face,
+                                                              int parity) {
+  __shared__ StepPlan sp;
+  const LatticeDesc L = lats[m];
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(L.plan);
+  uint32_t* dst = reinterpret_cast<uint32_t*>(&sp);
+  for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += blockDim.x) dst[w] = src[w];
+  __syncthreads();
+  zero_gradient_face<S, R>(static_cast<S*>(L.f[L.cur ^ parity]), L.flags, sp, face);
+}
+
+static int zero_gradient_blocks(int nx, int ny, int nz, int face) {
+  const int axis = face / 2;
+  const int64_t nodes = int64_t(axis == 0 ? ny : nx) * (axis == 2 ? ny : nz);
+  return int(std::min<int64_t>((nodes + 255) / 256, 4 * 148));
+}
+
+cudaError_t launch_zero_gradient(int prec, const StepPlan& p, void* fin, const int8_t* flags, int face, cudaStream_t s) {
+  const int blocks = zero_gradient_blocks(p.nx, p.ny, p.nz, face);
+  switch (prec) {
+    case 2: k_zero_gradient<float, float><<<blocks, 256, 0, s>>>(static_cast<float*>(fin), flags, p, face); break;
+    case 3: k_zero_gradient<__half, float><<<blocks, 256, 0, s>>>(static_cast<__half*>(fin), flags, p, face); break;
+    case 4: k_zero_gradient<__nv_bfloat16, float><<<blocks, 256, 0, s>>>(static_cast<__nv_bfloat16*>(fin), flags, p, face); break;
+    default: k_zero_gradient<double, double><<<blocks, 256, 0, s>>>(static_cast<double*>(fin), flags, p, face); break;
+  }
+  return cudaGetLastError();
+}
+
 cudaError_t launch_zero_gradient(int prec, const LatticeDesc* lats, int m, int face, int parity, const int n[3],
                                  cudaStream_t s) {
-  const int axis = face / 2;
-  const int64_t nodes = int64_t(axis == 0 ? n[1] : n[0]) * (axis == 2 ? n[1] : n[2]);
-  const int blocks = int(std::min<int64_t>((nodes + 255) / 256, 4 * 148));
+  const int blocks = zero_gradient_blocks(n[0], n[1], n[2], face);
   switch (prec) {
-    case 2: k_zero_gradient<float, float><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
-    case 3: k_zero_gradient<__half, float><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
-    case 4: k_zero_gradient<__nv_bfloat16, float><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
-    default: k_zero_gradient<double, double><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
+    case 2: k_zero_gradient_member<float, float><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
+    case 3: k_zero_gradient_member<__half, float><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
+    case 4: k_zero_gradient_member<__nv_bfloat16, float><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
+    default: k_zero_gradient_member<double, double><<<blocks, 256, 0, s>>>(lats, m, face, parity); break;
   }
   return cudaGetLastError();
 }

@@ -19,6 +19,7 @@ cudaError_t launch_set_distribution(int prec, void* f, const StepPlan& p, const 
 cudaError_t launch_double_couette(int prec, void* f, const StepPlan& p, int dim, const double uc[3],
                                   const double du[3], cudaStream_t s);
 struct LatticeDesc;
+cudaError_t launch_zero_gradient(int prec, const StepPlan& p, void* fin, const int8_t* flags, int face, cudaStream_t s);
 cudaError_t launch_zero_gradient(int prec, const LatticeDesc* lats, int m, int face, int parity, const int n[3],
                                  cudaStream_t s);
 cudaError_t launch_rasterize(int8_t* flags, const StepPlan& p, const int lo[3], const int hi[3], double dx,

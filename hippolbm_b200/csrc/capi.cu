@@ -149,8 +149,9 @@ struct hlbm_ctx {
   int64_t launches = 0;
   int64_t ncell = 0, stride = 0;
   StepPlan plan;
-  bool plan_dirty = true;
-  // pipelined persistent kernel: plan and lattice descriptor in device memory, tile list
+  bool plan_dirty = true;    // the operators or parameters changed after the plan was compiled
+  bool device_dirty = true;  // the plan changed after its device side (upload_plan) was last brought up to date
+  // plan and lattice descriptor in device memory (resident and batched launches), tile list of the pipelined kernel
   StepPlan* plan_dev = nullptr;
   LatticeDesc* desc_dev = nullptr;
   Tile* tiles_dev = nullptr;
@@ -297,21 +298,6 @@ bool pipeline_geometry(int nx, int ny, size_t es, int& rows, int& stages1, int& 
 // Tile list and stage geometry of the pipelined kernel (lbm_step_tma.cuh).
 int setup_pipeline(hlbm_ctx* c) {
   const StepPlan& p = c->plan;
-  if (!c->plan_dev) {
-    if (pool_alloc((void**)&c->plan_dev, sizeof(StepPlan), c->device, c->stream) != cudaSuccess ||
-        pool_alloc((void**)&c->desc_dev, sizeof(LatticeDesc), c->device, c->stream) != cudaSuccess ||
-        pool_alloc((void**)&c->group_dev, 256, c->device, c->stream) != cudaSuccess)
-      return fail(HLBM_ENOMEM, "cannot allocate the step plan");
-    HLBM_CK(cudaMemsetAsync(c->group_dev, 0, 256, c->stream));
-  }
-  HLBM_CK(cudaMemcpyAsync(c->plan_dev, &p, sizeof(StepPlan), cudaMemcpyHostToDevice, c->stream));
-  LatticeDesc d{};
-  d.plan = c->plan_dev;
-  d.f[0] = c->f[0];
-  d.f[1] = c->f[1];
-  d.flags = c->flags;
-  d.cur = 0;
-  HLBM_CK(cudaMemcpyAsync(c->desc_dev, &d, sizeof(d), cudaMemcpyHostToDevice, c->stream));
   c->tma_stages = 0;
   c->tma_stages2 = 0;
   const size_t es = elem_size(c->precision);
@@ -337,7 +323,8 @@ int setup_pipeline(hlbm_ctx* c) {
   return HLBM_OK;
 }
 
-int build_plan(hlbm_ctx* c) {
+// The step plan from the recorded operators and parameters: host work alone.
+int compile_plan(hlbm_ctx* c) {
   if (!c->plan_dirty) return HLBM_OK;
   StepPlan& p = c->plan;
   base_plan(c, p);
@@ -424,27 +411,62 @@ int build_plan(hlbm_ctx* c) {
     b.value = h.value;
   }
   p.face_mask = face_pass_mask(p, int(elem_size(c->precision)));
+  const int bytes = int(elem_size(c->precision));
+  if (!c->variant_tuned && bytes == 2)
+    c->variant = pipeline_kind(p, 9, bytes) == 2 && spans_avoided(p) ? 4 : 9;
+  c->plan_dirty = false;
+  c->device_dirty = true;
+  c->plan_version++;
+  return HLBM_OK;
+}
+
+// The plan's device side: its copy, the near-wall list and the tile list.  It copies and synchronises, so
+// steps that a caller captures do without it (hlbm_step): their launches carry the plan as a
+// parameter, and a copy captured in its place would leave the device side to the graph's replays.
+int upload_plan(hlbm_ctx* c) {
+  if (!c->device_dirty) return HLBM_OK;
+  StepPlan& p = c->plan;
   if (p.walls && p.wall_flags && p.ncell <= int64_t(0xffffffffu)) {
     if (int rc = refresh_near_list(c)) return rc;
     p.near_list = c->near_list;
     p.near_count = c->near_count;
   }
-  const int bytes = int(elem_size(c->precision));
-  if (!c->variant_tuned && bytes == 2)
-    c->variant = pipeline_kind(p, 9, bytes) == 2 && spans_avoided(p) ? 4 : 9;
+  HLBM_CK(cudaMemcpyAsync(c->plan_dev, &p, sizeof(StepPlan), cudaMemcpyHostToDevice, c->stream));
   if (int rc = setup_pipeline(c)) return rc;
-  c->plan_dirty = false;
-  c->plan_version++;
+  c->device_dirty = false;
   return HLBM_OK;
 }
 
+int build_plan(hlbm_ctx* c) {
+  if (int rc = compile_plan(c)) return rc;
+  return upload_plan(c);
+}
+
+// Whether a fused step of `variant` pulls without a wall test and leaves the nodes of the near-wall list to
+// the fix-up (launch.cuh: launch_step).
+bool walks_near_list(const hlbm_ctx* c, int variant) {
+  const StepPlan& p = c->plan;
+  const int bytes = int(elem_size(c->precision));
+  if (!p.walls || !p.wall_flags) return false;
+  if (rows_runs(p, variant, MODE_FUSED, bytes)) return true;
+  if (variant >= 8) variant = 5;
+  return variant < 6 && variant % 2 == 1 && vec_eligible_bytes(p, p.walls, bytes, variant);
+}
+
+// The kernel that steps lattice c inside a caller's capture: that of its variant, unless that one needs a
+// device side that cannot be brought up to date there (the pipelined kernel's tiles), or the near-wall
+// list, which a later change of the flags would take from under the graph's replays.
+int captured_variant(const hlbm_ctx* c) {
+  const bool tiles = c->variant == 6 || c->variant == 7;
+  return (tiles && c->device_dirty) || walks_near_list(c, c->variant) ? 4 : c->variant;
+}
+
 // the zero-gradient outlet passes of a plan: every pull of a step (or a read-out) sees them
-cudaError_t outlet_passes(int prec, const StepPlan& p, const LatticeDesc* descs, int m, int parity, const int n[3],
-                          cudaStream_t s, int64_t& launches) {
+cudaError_t outlet_passes(int prec, const StepPlan& p, void* fin, const int8_t* flags, cudaStream_t s, int64_t& launches) {
   for (int o = 0; o < p.nops; o++) {
     if (p.ops[o].kind != OP_ZERO_GRADIENT) continue;
     launches++;
-    if (cudaError_t e = launch_zero_gradient(prec, descs, m, p.ops[o].face, parity, n, s)) return e;
+    if (cudaError_t e = launch_zero_gradient(prec, p, fin, flags, p.ops[o].face, s)) return e;
   }
   return cudaSuccess;
 }
@@ -502,10 +524,8 @@ int resident_steps(hlbm_ctx* c, int64_t nsteps) {
 // kernel of `variant`.
 cudaError_t launch_with_plan(hlbm_ctx* c, int mode, const void* fin, void* fout, const StepPlan& p, int variant,
                              cudaStream_t s) {
-  if (mode != MODE_PROLOGUE)  // the descriptor holds f[0], f[1] with cur = 0
-    if (cudaError_t e = outlet_passes(c->precision, p, c->desc_dev, 0, fin == c->f[0] ? 0 : 1, c->n, s,
-                                      c->launches))
-      return e;
+  if (mode != MODE_PROLOGUE)
+    if (cudaError_t e = outlet_passes(c->precision, p, const_cast<void*>(fin), c->flags, s, c->launches)) return e;
   const int walls = p.walls;
   TmaArgs t;
   t.desc = c->desc_dev;
@@ -696,10 +716,21 @@ int hlbm_domain(const int32_t cell_dims[3], const double bmin[3], const double b
   if (pool_alloc((void**)&c->flags, flag_bytes, c->device, c->stream) != cudaSuccess ||
       pool_alloc((void**)&c->nearwall, flag_bytes, c->device, c->stream) != cudaSuccess ||
       pool_alloc((void**)&c->partials, sizeof(double) * 4 * 148 * 8, c->device, c->stream) != cudaSuccess ||
-      pool_alloc((void**)&c->stats_dev, sizeof(double) * 4, c->device, c->stream) != cudaSuccess) {
+      pool_alloc((void**)&c->stats_dev, sizeof(double) * 4, c->device, c->stream) != cudaSuccess ||
+      pool_alloc((void**)&c->plan_dev, sizeof(StepPlan), c->device, c->stream) != cudaSuccess ||
+      pool_alloc((void**)&c->desc_dev, sizeof(LatticeDesc), c->device, c->stream) != cudaSuccess ||
+      pool_alloc((void**)&c->group_dev, 256, c->device, c->stream) != cudaSuccess) {
     cudaGetLastError();
     return cleanup(fail(HLBM_ENOMEM, "hlbm_domain: cannot allocate flags"));
   }
+  LatticeDesc desc{};  // cur = 0: a launch's parity says which buffer is read
+  desc.plan = c->plan_dev;
+  desc.f[0] = c->f[0];
+  desc.f[1] = c->f[1];
+  desc.flags = c->flags;
+  if (cudaMemcpyAsync(c->desc_dev, &desc, sizeof(desc), cudaMemcpyHostToDevice, c->stream) != cudaSuccess ||
+      cudaMemsetAsync(c->group_dev, 0, 256, c->stream) != cudaSuccess)
+    return cleanup(fail(HLBM_ECUDA, "hlbm_domain: cannot set up the descriptor"));
   // init_obst: every flag FLUIDE_ (-1 = 0xff)
   if (cudaMemsetAsync(c->flags, 0xff, flag_bytes, c->stream) != cudaSuccess ||
       cudaMemsetAsync(c->nearwall, 0, flag_bytes, c->stream) != cudaSuccess)
@@ -1004,14 +1035,15 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
   if (!c || nsteps < 0) return fail(HLBM_EINVAL, "hlbm_step: bad argument");
   if (nsteps == 0) return HLBM_OK;
   if (int rc = set_device(c)) return rc;
-  if (int rc = build_plan(c)) return rc;
   // a caller's graph holds plain launches: no cooperative one, no overlapped ones
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
   HLBM_CK(cudaStreamIsCapturing(c->stream, &capture));
   const bool captured = capture != cudaStreamCaptureStatusNone;
+  if (int rc = captured ? compile_plan(c) : build_plan(c)) return rc;
+  const int variant = captured ? captured_variant(c) : c->variant;
   if (c->phase == MATER) c->phase = POSTCOL;
   if (c->phase == RAW) {
-    HLBM_CK(launch_step_kernel(c, MODE_PROLOGUE, c->f[c->cur], c->f[1 - c->cur]));
+    HLBM_CK(launch_step_variant(c, MODE_PROLOGUE, c->f[c->cur], c->f[1 - c->cur], variant));
     c->cur = 1 - c->cur;
     c->phase = POSTCOL;
     c->steps++;
@@ -1021,7 +1053,7 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
   // The call's first step is launched plainly, and the ones after it may overlap the kernel before them: that is
   // then one of this call's own, which write populations only (pdl_begin).
   for (int64_t s = 0; s < nsteps; s++) {
-    const cudaError_t e = launch_step_kernel(c, MODE_FUSED, c->f[c->cur], c->f[1 - c->cur]);
+    const cudaError_t e = launch_step_variant(c, MODE_FUSED, c->f[c->cur], c->f[1 - c->cur], variant);
     c->plan.overlap = 0;
     HLBM_CK(e);
     c->plan.overlap = !captured && s + 1 < nsteps;
@@ -1068,8 +1100,8 @@ int hlbm_simulation_state(hlbm_ctx* c, double out[3]) {
   if (int rc = set_device(c)) return rc;
   if (c->phase == POSTCOL) {  // straight from the post-collision state; the idle buffer stays idle
     if (int rc = build_plan(c)) return rc;
-    const void* fin = c->f[c->cur];
-    HLBM_CK(outlet_passes(c->precision, c->plan, c->desc_dev, 0, fin == c->f[0] ? 0 : 1, c->n, c->stream, c->launches));
+    void* fin = c->f[c->cur];
+    HLBM_CK(outlet_passes(c->precision, c->plan, fin, c->flags, c->stream, c->launches));
     c->launches++;
     HLBM_CK(observe_state(c, fin));
   } else {
@@ -1679,9 +1711,12 @@ cudaError_t batch_launch(hlbm_batch* b, int parity) {
   for (size_t m = 0; m < b->members.size(); m++) {  // members that pull this launch (not fresh)
     hlbm_ctx* c = b->members[m];
     if (c->phase == RAW) continue;
-    if (cudaError_t e = outlet_passes(b->precision, c->plan, b->desc_dev, int(m), parity, c->n, b->stream,
-                                      b->launches))
-      return e;
+    for (int o = 0; o < c->plan.nops; o++) {
+      if (c->plan.ops[o].kind != OP_ZERO_GRADIENT) continue;
+      b->launches++;
+      if (cudaError_t e = launch_zero_gradient(b->precision, b->desc_dev, int(m), c->plan.ops[o].face, parity, c->n, b->stream))
+        return e;
+    }
   }
   StepPlan dummy;
   std::memset(&dummy, 0, sizeof(dummy));
@@ -1884,8 +1919,7 @@ int hlbm_batch_autotune(hlbm_batch* b, int32_t reps, int32_t* chosen, double* ms
       for (hlbm_ctx* c : b->members) {
         if (e == cudaSuccess && !c->join_ev) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, b->fork_ev, 0);
-        StepPlan pk = c->plan;
-          if (e == cudaSuccess)
+        if (e == cudaSuccess)
           e = launch_with_plan(c, c->phase == RAW ? MODE_PROLOGUE : MODE_FUSED, c->f[c->cur], c->f[1 - c->cur],
                                c->plan, concurrent_variant(c), c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(c->join_ev, c->stream);
