@@ -373,28 +373,40 @@ __device__ __forceinline__ void macro(const R (&v)[Q], R& rho, R& ux, R& uy, R& 
 }
 
 // ------------------------------------------------------------------ BGK (bgk.hpp:47-62)
+// Strict: the reference's operation order, compiled without contraction.  Otherwise every fused
+// multiply-add is written out: the compiler's own choice (which of two products of u^2 to fuse) differed
+// between kernels, so that the same lattice with walls ended in other last bits by the resident
+// kernel than by the one-node kernel.
 template <typename R, bool STRICT>
 __device__ __forceinline__ void bgk(R (&v)[Q], const StepPlan& p) {
   R rho, ux, uy, uz;
   macro<R, STRICT>(v, rho, ux, uy, uz);
-  const R u_squ = (ux * ux + uy * uy + uz * uz);
-  const R tau = R(p.tau), inv_tau = R(p.inv_tau);
   const R Fx = R(p.F[0]), Fy = R(p.F[1]), Fz = R(p.F[2]);
   const bool force = p.has_force != 0;
-  Unroll<0, Q>::run([&]<int I>() {
-    constexpr R w = weight<R, I>();
-    const R eu = edot<I, R>(ux, uy, uz);
-    const R feq = w * rho * (R(1.) + R(3.) * eu + R(4.5) * eu * eu - R(1.5) * u_squ);
-    if (STRICT) {
+  if constexpr (STRICT) {
+    const R u_squ = (ux * ux + uy * uy + uz * uz);
+    const R tau = R(p.tau);
+    Unroll<0, Q>::run([&]<int I>() {
+      constexpr R w = weight<R, I>();
+      const R eu = edot<I, R>(ux, uy, uz);
+      const R feq = w * rho * (R(1.) + R(3.) * eu + R(4.5) * eu * eu - R(1.5) * u_squ);
       R d = (feq - v[I]) / tau;
       if (force) d = d + R(3.) * rho * w * edot<I, R>(Fx, Fy, Fz);
       v[I] = v[I] + d;
-    } else {
-      R d = (feq - v[I]) * inv_tau;
-      if (force) d += R(3.) * rho * w * edot<I, R>(Fx, Fy, Fz);
-      v[I] += d;
-    }
-  });
+    });
+  } else {
+    static_assert(sizeof(R) == 8, "the other tiers collide by bgk_v");
+    const R u_squ = __fma_rn(uz, uz, __fma_rn(uy, uy, __dmul_rn(ux, ux)));
+    const R inv_tau = R(p.inv_tau);
+    Unroll<0, Q>::run([&]<int I>() {
+      constexpr R w = weight<R, I>();
+      const R eu = edot<I, R>(ux, uy, uz);
+      const R poly = __fma_rn(R(-1.5), u_squ, __fma_rn(__dmul_rn(R(4.5), eu), eu, __fma_rn(R(3.), eu, R(1.))));
+      R d = __dmul_rn(__fma_rn(__dmul_rn(w, rho), poly, -v[I]), inv_tau);
+      if (force) d = __fma_rn(__dmul_rn(__dmul_rn(R(3.), rho), w), edot<I, R>(Fx, Fy, Fz), d);
+      v[I] = __dadd_rn(v[I], d);
+    });
+  }
 }
 
 // ------------------------------------------------------------------ MRT (mrt.hpp:42-193)
