@@ -129,7 +129,7 @@ struct hlbm_ctx {
   int cur = 0;
   int8_t* flags = nullptr;
   int8_t* nearwall = nullptr;  // per node: 1 some pull comes from a wall node, 2 a wall node (k_near_wall)
-  uint32_t* near_list = nullptr;  // the nodes marked 1, for plans with wall_bounce_back; built with the plan
+  uint32_t* near_list = nullptr;  // the nodes marked 1, for kernels that walk them (near_list_for)
   int32_t near_count = 0;
   bool near_stale = true;         // the map changed after the list was built
   bool maybe_walls = false;     // the flags may hold wall nodes (an obstacle was rasterised or put)
@@ -213,8 +213,8 @@ int refresh_near_wall(hlbm_ctx* c) {
 }
 
 // The list of the near-wall nodes (k_near_list), which the fix-up walks: a sphere of radius
-// 20 leaves 7 k of 2.4 M nodes to look at.  Counted, allocated and filled when a
-// plan with wall_bounce_back is built after the flags changed.
+// 20 leaves 7 k of 2.4 M nodes to look at.  Counted, allocated and filled before the first step by a kernel
+// that needs it after the flags changed (near_list_for): two passes over the map and a wait for the count.
 int refresh_near_list(hlbm_ctx* c) {
   if (!c->near_stale) return HLBM_OK;
   pool_free(c->near_list, c->stream);
@@ -420,18 +420,12 @@ int compile_plan(hlbm_ctx* c) {
   return HLBM_OK;
 }
 
-// The plan's device side: its copy, the near-wall list and the tile list.  It copies and synchronises, so
-// steps that a caller captures do without it (hlbm_step): their launches carry the plan as a
-// parameter, and a copy captured in its place would leave the device side to the graph's replays.
+// The plan's device side: its copy and the tile list.  It copies and synchronises, so steps that a caller
+// captures do without it (hlbm_step): their launches carry the plan as a parameter, and a copy
+// captured in its place would leave the device side to the graph's replays.
 int upload_plan(hlbm_ctx* c) {
   if (!c->device_dirty) return HLBM_OK;
-  StepPlan& p = c->plan;
-  if (p.walls && p.wall_flags && p.ncell <= int64_t(0xffffffffu)) {
-    if (int rc = refresh_near_list(c)) return rc;
-    p.near_list = c->near_list;
-    p.near_count = c->near_count;
-  }
-  HLBM_CK(cudaMemcpyAsync(c->plan_dev, &p, sizeof(StepPlan), cudaMemcpyHostToDevice, c->stream));
+  HLBM_CK(cudaMemcpyAsync(c->plan_dev, &c->plan, sizeof(StepPlan), cudaMemcpyHostToDevice, c->stream));
   if (int rc = setup_pipeline(c)) return rc;
   c->device_dirty = false;
   return HLBM_OK;
@@ -451,6 +445,15 @@ bool walks_near_list(const hlbm_ctx* c, int variant) {
   if (rows_runs(p, variant, MODE_FUSED, bytes)) return true;
   if (variant >= 8) variant = 5;
   return variant < 6 && variant % 2 == 1 && vec_eligible_bytes(p, p.walls, bytes, variant);
+}
+
+// The near-wall list in the plan, up to date, if a fused step of `variant` walks it.
+int near_list_for(hlbm_ctx* c, int variant) {
+  if (!walks_near_list(c, variant)) return HLBM_OK;
+  if (int rc = refresh_near_list(c)) return rc;
+  c->plan.near_list = c->near_list;
+  c->plan.near_count = c->near_count;
+  return HLBM_OK;
 }
 
 // The kernel that steps lattice c inside a caller's capture: that of its variant, unless that one needs a
@@ -1049,7 +1052,10 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
     c->steps++;
     nsteps--;
   }
-  if (nsteps > 0 && !captured && resident_applies(c)) return resident_steps(c, nsteps);
+  if (nsteps > 0 && !captured) {
+    if (resident_applies(c)) return resident_steps(c, nsteps);
+    if (int rc = near_list_for(c, variant)) return rc;
+  }
   // The call's first step is launched plainly, and the ones after it may overlap the kernel before them: that is
   // then one of this call's own, which write populations only (pdl_begin).
   for (int64_t s = 0; s < nsteps; s++) {
@@ -1416,6 +1422,11 @@ int hlbm_autotune(hlbm_ctx* c, int32_t reps, int32_t* chosen, double* ms_per_var
     if (v < 6 && (v % 2) == 1 && !vec_applies(c, v)) continue;
     if (v >= 8 && !rows_runs(c->plan, v, MODE_FUSED, int(elem_size(c->precision)))) continue;
     if ((v == 6 || v == 7) && c->tma_stages < 2) continue;
+    if (int rc = near_list_for(c, v)) {
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      return rc;
+    }
     cudaError_t e = launch_step_variant(c, MODE_FUSED, fin, fout, v);  // warm-up
     if (e == cudaSuccess) e = cudaEventRecord(e0, c->stream);
     for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch_step_variant(c, MODE_FUSED, fin, fout, v);
@@ -1557,6 +1568,7 @@ int batch_step_concurrent(hlbm_batch* b, int64_t nsteps) {
   bool fresh = false;
   for (hlbm_ctx* c : b->members) {
     if (int rc = build_plan(c)) return rc;
+    if (int rc = near_list_for(c, concurrent_variant(c))) return rc;
     if (c->phase == MATER) c->phase = POSTCOL;
     fresh |= c->phase == RAW;
     HLBM_CK(cudaStreamSynchronize(c->stream));
@@ -1876,6 +1888,7 @@ int hlbm_batch_autotune(hlbm_batch* b, int32_t reps, int32_t* chosen, double* ms
   HLBM_CK(cudaSetDevice(b->device));
   for (hlbm_ctx* c : b->members) {
     if (int rc = build_plan(c)) return rc;
+    if (int rc = near_list_for(c, concurrent_variant(c))) return rc;
     if (c->phase == MATER) c->phase = POSTCOL;  // the state is the post-collision one either way
     HLBM_CK(cudaStreamSynchronize(c->stream));
   }
