@@ -501,17 +501,16 @@ cudaError_t launch_resident_tier(int precision, const ResidentArgs& a, int walls
 constexpr int RESIDENT_STEPS = 1024;
 int resident_steps(hlbm_ctx* c, int64_t nsteps) {
   ResidentArgs a;
-  a.descs = c->desc_dev;
+  a.desc = c->desc_dev;
   a.left = c->group_dev;
-  a.bars = c->group_dev + RES_BAR_STRIDE;
-  a.nbars = 1;
+  a.bar = c->group_dev + RES_BAR_STRIDE;
   a.err = c->err_dev;
   a.grid = int(std::min<int64_t>(c->sms, (c->ncell + 63) / 64));
   // the caller's bound in the tiers whose default kernels always waited (hlbm_set_wait_limit)
   a.wait_limit = elem_size(c->precision) == 2 ? c->wait_limit : TMA_WAIT_LIMIT;
   while (nsteps > 0) {
     const int m = int(std::min<int64_t>(nsteps, RESIDENT_STEPS));
-    a.one = ResidentTask{0, 0, a.grid, 0, m};
+    a.nsteps = m;
     a.parity = c->cur;  // the descriptor holds f[0], f[1] with cur = 0
     a.seed = uint32_t(c->steps);
     c->launches++;

@@ -3,14 +3,13 @@
 //
 // What bounds a small lattice stepped launch by launch is not its bytes: each launch starts with
 // cold instruction and constant caches, runs one latency chain (index arithmetic, one round of
-// loads, one collision, one round of stores) and drains, and the tiers with a face pass do that
-// twice a step.  Here one cooperative launch takes many steps: the CTAs of a group own one
-// lattice, every thread steps its share of the nodes, and a group barrier (a counter in
-// global memory) separates the steps.  A launch takes a list of such tasks (a lattice and its CTAs);
-// a lattice stepped alone is one task.  Measured (us a step): FP64 31^3 6.3 -> 3.5, FP32 24^3 11.4 ->
-// 2.6, FP16 24^3 20.6 -> 3.1, BF16 57 x 43 x 61 20 -> 8.4; the barrier alone takes 1.2 of them.
+// loads, one collision, one round of stores) and drains, and the tiers with a fix-up launch do that
+// twice a step.  Here one cooperative launch takes many steps: its CTAs step the lattice's nodes and a
+// barrier (a counter in global memory) separates the steps.  Measured (us a step): FP64 31^3
+// 6.3 -> 3.5, FP32 24^3 11.4 -> 2.6, FP16 24^3 20.6 -> 3.1, BF16 57 x 43 x 61 20 -> 8.4; the barrier alone
+// takes 1.2 of them.
 //
-// A lattice of no more nodes than the group has threads gets one node per thread for the whole launch,
+// A lattice of no more nodes than the launch has threads gets one node per thread for the whole launch,
 // whose addresses to pull from are computed once.  Larger ones (16-bit tiers) work through items, whole
 // warps of one kind:
 //   faces     the nodes on the lattice's faces, each once, by the general one-node gather (periodic
@@ -20,12 +19,10 @@
 //             on a face stores its other half alone), so the stored bits are the same.
 // Warps are dealt out across the CTAs first, so a lattice of few items still uses every SM.
 //
-// The buffers change hands between SMs inside the launch, so populations are read past L1 (ld.cg);
+// The buffers change hands between SMs inside the launch, so populations are read past L1 (ld_l2);
 // flags and the near-wall map do not change and go through it.  Every wait is bounded by wait_limit
-// polls and two seconds, after which the kernel records an error and returns; the host cuts long
-// runs into launches of some 50 ms.  A cooperative launch keeps all CTAs resident, so a group's CTAs
-// always run together; every CTA takes its tasks in list order, so groups that share CTAs cannot
-// wait for one another in a cycle.
+// polls and two seconds, after which the kernel records an error and returns.  A cooperative launch
+// starts only when all its CTAs are resident, so they can wait for one another.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -35,23 +32,15 @@
 namespace hlbm {
 
 constexpr int RES_THREADS = 512;      // one CTA per SM, 128 registers a thread
-constexpr int RES_BAR_STRIDE = 32;    // the tasks' barrier counters lie 128 bytes apart
-
-// `nsteps` steps of one lattice for the CTAs [first, first + ctas), which meet at the counter `bar`.
-struct ResidentTask {
-  int32_t lat, first, ctas, bar, nsteps;
-};
+constexpr int RES_BAR_STRIDE = 32;    // the barrier's counter lies 128 bytes past the count of CTAs that have left
 
 struct ResidentArgs {
-  LatticeDesc* descs = nullptr;
-  const ResidentTask* tasks = nullptr;  // null: `one` alone
-  int ntasks = 1;
-  ResidentTask one{};
-  int parity = 0;        // f[cur ^ parity] is read first
-  long long seed = -1;   // step number of a single lattice; -1: the descriptors' counters
-  unsigned* left = nullptr;  // CTAs that have left the launch; zero between launches
-  unsigned* bars = nullptr;  // the tasks' barrier counters, zero between launches
-  int nbars = 0;
+  const LatticeDesc* desc = nullptr;
+  int nsteps = 0;
+  int parity = 0;              // f[cur ^ parity] is read first
+  uint32_t seed = 0;           // step number of the first step
+  unsigned* left = nullptr;    // CTAs that have left the launch; zero between launches
+  unsigned* bar = nullptr;     // the barrier's counter, zero between launches
   int* err = nullptr;
   int grid = 0;
   long long wait_limit = TMA_WAIT_LIMIT;
@@ -69,7 +58,7 @@ inline bool resident_plan(const StepPlan& p) {
 __host__ __device__ inline uint64_t res_magic(uint64_t d) { return d <= 1 ? 0 : ~uint64_t(0) / d + 1; }
 __device__ __forceinline__ uint32_t res_div(uint32_t n, uint64_t m) { return m == 0 ? n : uint32_t(__umul64hi(uint64_t(n), m)); }
 
-// What the threads of a group need of a lattice besides its plan, staged in shared memory.
+// What the threads need of a lattice besides its plan, staged in shared memory.
 struct ResidentGeometry {
   int off[Q];                      // element offset of direction I's source from the node's index
   uint32_t z_nodes, y_nodes, nface, nface_pad, nitems;  // face nodes in the z planes, then the y rows; all; padded
@@ -238,92 +227,85 @@ __device__ __forceinline__ void resident_pair(const S* fin, S* fout, const int8_
 
 template <typename S, typename R, bool STRICT, bool WALLS>
 __global__ void __launch_bounds__(RES_THREADS, 1)
-    k_step_resident(const LatticeDesc* __restrict__ lats, const ResidentTask* __restrict__ tasks, int ntasks,
-                    const ResidentTask one, int parity, long long seed, unsigned* left, unsigned* bars, int nbars, int* err, long long wait_limit) {
+    k_step_resident(const LatticeDesc* __restrict__ desc, int nsteps, int parity, uint32_t seed, unsigned* left,
+                    unsigned* bar, int* err, long long wait_limit) {
   __shared__ StepPlan p;
   __shared__ ResidentGeometry g;
   __shared__ int bail;
-  if (threadIdx.x == 0) bail = 0;
-  const int cta = blockIdx.x;
-  for (int t = 0; t < ntasks; t++) {
-    const ResidentTask tk = tasks ? tasks[t] : one;
-    if (cta < tk.first || cta >= tk.first + tk.ctas) continue;
-    const LatticeDesc L = lats[tk.lat];
-    __syncthreads();  // the previous task's plan is no longer read
-    const uint32_t* src = reinterpret_cast<const uint32_t*>(L.plan);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(&p);
-    for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += blockDim.x) dst[w] = src[w];
-    __syncthreads();
-    const bool pairs = is_16bit<S>() && p.nsets == 0 && (!p.wall_flags || p.walls);
-    if (threadIdx.x == 0) {
-      resident_geometry(p, pairs, is_16bit<S>() && !pairs, g);
-      p.seed = seed >= 0 ? uint32_t(seed) : L.step[parity];
-    }
-    __syncthreads();
-    const bool walls = WALLS && p.walls;
-    const uint32_t nthreads = uint32_t(tk.ctas) * RES_THREADS;
-    const uint32_t me = ((threadIdx.x >> 5) * uint32_t(tk.ctas) + uint32_t(cta - tk.first)) * 32 + (threadIdx.x & 31);
-    const int cur0 = L.cur ^ parity;
-    auto step_done = [&](int k) {  // false when the launch gives up
-      if (k + 1 == tk.nsteps) return true;
-      if (!group_barrier(bars + tk.bar, unsigned(tk.ctas) * unsigned(k + 1), wait_limit, err, &bail)) return false;
-      if (threadIdx.x == 0) p.seed++;
-      __syncthreads();
-      return true;
-    };
-    bool ok = true;
-    if (uint32_t(p.ncell) <= nthreads) {
-      // one node per thread for the whole launch: where it pulls from stays in registers
-      ResidentNode it;
-      int src[Q];
-      S raw[Q];
-      const bool live = me < uint32_t(p.ncell);
-      bool edge = false;
-      if (live) {
-        it.idx = me;
-        it.z = int(res_div(me, g.m_plane));
-        const uint32_t rem = me - uint32_t(it.z) * uint32_t(p.nx) * uint32_t(p.ny);
-        it.y = int(res_div(rem, g.m_nx));
-        it.x = int(rem - uint32_t(it.y) * uint32_t(p.nx));
-        it.flag = L.flags[me];
-        resident_sources<WALLS>(L.flags, p, walls, it, src);
-        edge = on_op_face(p, it.x, it.y, it.z);
-      }
-      for (int k = 0; k < tk.nsteps && ok; k++) {
-        const S* fin = static_cast<const S*>(L.f[cur0 ^ (k & 1)]);
-        S* fout = static_cast<S*>(L.f[cur0 ^ (k & 1) ^ 1]);
-        if (live) {
-          Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<true>(fin + src[I]); });
-          resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, edge);
-        }
-        ok = step_done(k);
-      }
-    } else if constexpr (is_16bit<S>()) {
-      for (int k = 0; k < tk.nsteps && ok; k++) {
-        const S* fin = static_cast<const S*>(L.f[cur0 ^ (k & 1)]);
-        S* fout = static_cast<S*>(L.f[cur0 ^ (k & 1) ^ 1]);
-        uint32_t i = me;
-        for (; i < g.nface_pad; i += nthreads) {
-          if (i >= g.nface) continue;
-          ResidentNode it;
-          S raw[Q];
-          resident_face<S, WALLS>(fin, L.flags, p, g, walls, !pairs, i, it, raw);
-          resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, on_op_face(p, it.x, it.y, it.z));
-        }
-        for (; i < g.nitems; i += nthreads)
-          resident_pair<S, WALLS>(fin, fout, L.flags, p, g, walls, g.pair_begin + 2 * (i - g.nface_pad));
-        ok = step_done(k);
-      }
-    }
-    if (!ok) break;
+  const LatticeDesc L = *desc;
+  const uint32_t* from = reinterpret_cast<const uint32_t*>(L.plan);
+  uint32_t* to = reinterpret_cast<uint32_t*>(&p);
+  for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += RES_THREADS) to[w] = from[w];
+  __syncthreads();
+  const bool pairs = is_16bit<S>() && p.nsets == 0 && (!p.wall_flags || p.walls);
+  if (threadIdx.x == 0) {
+    bail = 0;
+    resident_geometry(p, pairs, is_16bit<S>() && !pairs, g);
+    p.seed = seed;
   }
-  group_leave(left, bars, nbars);
+  __syncthreads();
+  const bool walls = WALLS && p.walls;
+  const uint32_t nthreads = gridDim.x * RES_THREADS;
+  const uint32_t me = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+  const int cur0 = L.cur ^ parity;
+  auto step_done = [&](int k) {  // false when the launch gives up
+    if (k + 1 == nsteps) return true;
+    if (!group_barrier(bar, gridDim.x * unsigned(k + 1), wait_limit, err, &bail)) return false;
+    if (threadIdx.x == 0) p.seed++;
+    __syncthreads();
+    return true;
+  };
+  bool ok = true;
+  if (uint32_t(p.ncell) <= nthreads) {
+    // one node per thread for the whole launch: where it pulls from stays in registers
+    ResidentNode it;
+    int src[Q];
+    S raw[Q];
+    const bool live = me < uint32_t(p.ncell);
+    bool edge = false;
+    if (live) {
+      it.idx = me;
+      it.z = int(res_div(me, g.m_plane));
+      const uint32_t rem = me - uint32_t(it.z) * uint32_t(p.nx) * uint32_t(p.ny);
+      it.y = int(res_div(rem, g.m_nx));
+      it.x = int(rem - uint32_t(it.y) * uint32_t(p.nx));
+      it.flag = L.flags[me];
+      resident_sources<WALLS>(L.flags, p, walls, it, src);
+      edge = on_op_face(p, it.x, it.y, it.z);
+    }
+    for (int k = 0; k < nsteps && ok; k++) {
+      const S* fin = static_cast<const S*>(L.f[cur0 ^ (k & 1)]);
+      S* fout = static_cast<S*>(L.f[cur0 ^ (k & 1) ^ 1]);
+      if (live) {
+        Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<true>(fin + src[I]); });
+        resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, edge);
+      }
+      ok = step_done(k);
+    }
+  } else if constexpr (is_16bit<S>()) {
+    for (int k = 0; k < nsteps && ok; k++) {
+      const S* fin = static_cast<const S*>(L.f[cur0 ^ (k & 1)]);
+      S* fout = static_cast<S*>(L.f[cur0 ^ (k & 1) ^ 1]);
+      uint32_t i = me;
+      for (; i < g.nface_pad; i += nthreads) {
+        if (i >= g.nface) continue;
+        ResidentNode it;
+        S raw[Q];
+        resident_face<S, WALLS>(fin, L.flags, p, g, walls, !pairs, i, it, raw);
+        resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, on_op_face(p, it.x, it.y, it.z));
+      }
+      for (; i < g.nitems; i += nthreads)
+        resident_pair<S, WALLS>(fin, fout, L.flags, p, g, walls, g.pair_begin + 2 * (i - g.nface_pad));
+      ok = step_done(k);
+    }
+  }
+  group_leave(left, bar);
 }
 
 template <typename S, typename R, bool STRICT>
 cudaError_t launch_resident(const ResidentArgs& a, int walls, cudaStream_t s) {
   ResidentArgs c = a;
-  void* args[] = {&c.descs, &c.tasks, &c.ntasks, &c.one, &c.parity, &c.seed, &c.left, &c.bars, &c.nbars, &c.err, &c.wait_limit};
+  void* args[] = {&c.desc, &c.nsteps, &c.parity, &c.seed, &c.left, &c.bar, &c.err, &c.wait_limit};
   const void* kern = walls ? (const void*)k_step_resident<S, R, STRICT, true> : (const void*)k_step_resident<S, R, STRICT, false>;
   return cudaLaunchCooperativeKernel(kern, dim3(c.grid), dim3(RES_THREADS), args, 0, s);
 }
