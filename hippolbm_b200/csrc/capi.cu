@@ -496,20 +496,21 @@ cudaError_t launch_resident_tier(int precision, const ResidentArgs& a, int walls
   }
 }
 
-// nsteps fused steps of one lattice in resident launches of at most RESIDENT_STEPS (a step of the
-// largest lattice taken is some 40 us, and the waits of a launch give up after two seconds)
-constexpr int RESIDENT_STEPS = 1024;
+// nsteps fused steps of one lattice in resident launches of about a millisecond, so that work of other
+// streams that finds no room beside one does not wait long: 256 steps of 3 to 5 us with one node per
+// thread, 64 of 8 to 21 us beyond.
 int resident_steps(hlbm_ctx* c, int64_t nsteps) {
   ResidentArgs a;
   a.desc = c->desc_dev;
   a.left = c->group_dev;
   a.bar = c->group_dev + RES_BAR_STRIDE;
   a.err = c->err_dev;
-  a.grid = int(std::min<int64_t>(c->sms, (c->ncell + 63) / 64));
+  resident_shape(c->ncell, c->sms, a.grid, a.threads);
+  const int64_t chunk = c->ncell <= int64_t(a.grid) * a.threads ? 256 : 64;
   // the caller's bound in the tiers whose default kernels always waited (hlbm_set_wait_limit)
   a.wait_limit = elem_size(c->precision) == 2 ? c->wait_limit : TMA_WAIT_LIMIT;
   while (nsteps > 0) {
-    const int m = int(std::min<int64_t>(nsteps, RESIDENT_STEPS));
+    const int m = int(std::min(nsteps, chunk));
     a.nsteps = m;
     a.parity = c->cur;  // the descriptor holds f[0], f[1] with cur = 0
     a.seed = uint32_t(c->steps);

@@ -17,7 +17,9 @@
 //   interior  the node pairs (n, n + 1), n even, of every other kernel, whose sources are idx - d_I: one
 //             offset per direction, packed FP32 and one 32-bit store per direction (a pair with one node
 //             on a face stores its other half alone), so the stored bits are the same.
-// Warps are dealt out across the CTAs first, so a lattice of few items still uses every SM.
+// Warps are dealt out across the CTAs first, so a lattice of few items still uses every SM; CTAs have no
+// more warps than that takes, so that the launches of several small lattices, each on its stream, share the
+// SMs (resident_shape).
 //
 // The buffers change hands between SMs inside the launch, so populations are read past L1 (ld_l2);
 // flags and the near-wall map do not change and go through it.  Every wait is bounded by wait_limit
@@ -26,12 +28,14 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "group_barrier.cuh"
 #include "lbm_step_vec.cuh"
 
 namespace hlbm {
 
-constexpr int RES_THREADS = 512;      // one CTA per SM, 128 registers a thread
+constexpr int RES_THREADS = 512;      // threads of a CTA at most: one CTA per SM, 128 registers a thread
 constexpr int RES_BAR_STRIDE = 32;    // the barrier's counter lies 128 bytes past the count of CTAs that have left
 
 struct ResidentArgs {
@@ -42,7 +46,7 @@ struct ResidentArgs {
   unsigned* left = nullptr;    // CTAs that have left the launch; zero between launches
   unsigned* bar = nullptr;     // the barrier's counter, zero between launches
   int* err = nullptr;
-  int grid = 0;
+  int grid = 0, threads = RES_THREADS;
   long long wait_limit = TMA_WAIT_LIMIT;
 };
 
@@ -52,6 +56,15 @@ inline bool resident_plan(const StepPlan& p) {
   for (int o = 0; o < p.nops; o++)
     if (p.ops[o].kind == OP_ZERO_GRADIENT) return false;
   return int64_t(Q) * p.stride < (int64_t(1) << 31);
+}
+
+// CTAs and threads of a launch.  A lattice with a thread for each node takes as many warps as it has, spread
+// over all SMs: as blocks of 512 threads it filled the register file of every SM with idle warps, and eight
+// FP64 24^3 lattices, each on its stream, took 3.2 us a lattice step, against 0.9 with the warps they need.
+inline void resident_shape(int64_t ncell, int sms, int& grid, int& threads) {
+  grid = int(std::min<int64_t>(sms, (ncell + 63) / 64));
+  const int64_t warps = (ncell + 32 * grid - 1) / (32 * int64_t(grid));
+  threads = 32 * int(std::min<int64_t>(RES_THREADS / 32, warps));
 }
 
 // floor(n / d) = umul64hi(n, m) for n < 2^32, m = ceil(2^64 / d); d = 1 is marked by m = 0
@@ -235,7 +248,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
   const LatticeDesc L = *desc;
   const uint32_t* from = reinterpret_cast<const uint32_t*>(L.plan);
   uint32_t* to = reinterpret_cast<uint32_t*>(&p);
-  for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += RES_THREADS) to[w] = from[w];
+  for (int w = threadIdx.x; w < int(sizeof(StepPlan) / 4); w += blockDim.x) to[w] = from[w];
   __syncthreads();
   const bool pairs = is_16bit<S>() && p.nsets == 0 && (!p.wall_flags || p.walls);
   if (threadIdx.x == 0) {
@@ -245,7 +258,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
   }
   __syncthreads();
   const bool walls = WALLS && p.walls;
-  const uint32_t nthreads = gridDim.x * RES_THREADS;
+  const uint32_t nthreads = gridDim.x * blockDim.x;
   const uint32_t me = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
   const int cur0 = L.cur ^ parity;
   auto step_done = [&](int k) {  // false when the launch gives up
@@ -307,7 +320,7 @@ cudaError_t launch_resident(const ResidentArgs& a, int walls, cudaStream_t s) {
   ResidentArgs c = a;
   void* args[] = {&c.desc, &c.nsteps, &c.parity, &c.seed, &c.left, &c.bar, &c.err, &c.wait_limit};
   const void* kern = walls ? (const void*)k_step_resident<S, R, STRICT, true> : (const void*)k_step_resident<S, R, STRICT, false>;
-  return cudaLaunchCooperativeKernel(kern, dim3(c.grid), dim3(RES_THREADS), args, 0, s);
+  return cudaLaunchCooperativeKernel(kern, dim3(c.grid), dim3(c.threads), args, 0, s);
 }
 
 // one entry per precision tier (defined in resident_*.cu)

@@ -207,8 +207,9 @@ int hlbm_info(hlbm_ctx* ctx, int64_t info[8]);
  * FP64 4, FP32 1, FP16 / BF16 9; 4 instead of 9 where rows are ragged and some face is no boundary
  * operator's) until hlbm_tune or hlbm_autotune chooses.  Until hlbm_tune chooses, hlbm_step advances
  * lattices that fit the GPU at one node per thread, and 16-bit BGK lattices of up to 50 MB, by many steps
- * a launch (not while the context's stream is being captured).  Variants 6, 7: persistent
- * kernel fed by bulk asynchronous copies of whole rows
+ * a launch of about a millisecond (not while the context's stream is being captured); such launches of
+ * lattices on different streams run side by side up to 64 k nodes together (on 148 SMs), and one after
+ * another beyond.  Variants 6, 7: persistent kernel fed by bulk asynchronous copies of whole rows
  * into shared-memory stages (256 or 512 threads per CTA; needs nx * bytes per population to be a
  * multiple of 16; otherwise variant 4 runs).  hlbm_autotune times `reps` fused launches of every
  * variant on this lattice (from the current populations into the idle buffer, so the state does
