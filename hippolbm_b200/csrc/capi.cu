@@ -23,6 +23,7 @@
 #include "host_copy.h"
 #include "launch.cuh"
 #include "lbm_step_resident.cuh"
+#include "many_steps.h"
 #include "observe.cuh"
 
 using namespace hlbm;
@@ -498,8 +499,8 @@ cudaError_t launch_resident_tier(int precision, const ResidentArgs& a, int walls
 
 // nsteps fused steps of one lattice in resident launches of about a millisecond, so that work of other
 // streams that finds no room beside one does not wait long: 256 steps of 3 to 5 us with one node per
-// thread, 64 of 8 to 21 us beyond.
-int resident_steps(hlbm_ctx* c, int64_t nsteps) {
+// thread, 64 of 8 to 21 us beyond.  `done`: fewer where the device refuses the launch (many_steps).
+int resident_steps(hlbm_ctx* c, int64_t nsteps, int64_t& done) {
   ResidentArgs a;
   a.desc = c->desc_dev;
   a.left = c->group_dev;
@@ -509,17 +510,18 @@ int resident_steps(hlbm_ctx* c, int64_t nsteps) {
   const int64_t chunk = c->ncell <= int64_t(a.grid) * a.threads ? 256 : 64;
   // the caller's bound in the tiers whose default kernels always waited (hlbm_set_wait_limit)
   a.wait_limit = elem_size(c->precision) == 2 ? c->wait_limit : TMA_WAIT_LIMIT;
-  while (nsteps > 0) {
-    const int m = int(std::min(nsteps, chunk));
+  const auto launch = [&](int m) {
     a.nsteps = m;
     a.parity = c->cur;  // the descriptor holds f[0], f[1] with cur = 0
     a.seed = uint32_t(c->steps);
+    const cudaError_t e = launch_resident_tier(c->precision, a, c->plan.walls, c->stream);
+    if (e != cudaSuccess) return e;
     c->launches++;
-    HLBM_CK(launch_resident_tier(c->precision, a, c->plan.walls, c->stream));
     if (m & 1) c->cur = 1 - c->cur;
     c->steps += m;
-    nsteps -= m;
-  }
+    return e;
+  };
+  HLBM_CK(many_steps(nsteps, chunk, done, launch, [] { cudaGetLastError(); }));
   return HLBM_OK;
 }
 
@@ -1053,7 +1055,12 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
     nsteps--;
   }
   if (nsteps > 0 && !captured) {
-    if (resident_applies(c)) return resident_steps(c, nsteps);
+    if (resident_applies(c)) {
+      int64_t done = 0;
+      if (int rc = resident_steps(c, nsteps, done)) return rc;
+      nsteps -= done;
+      if (nsteps == 0) return HLBM_OK;
+    }
     if (int rc = near_list_for(c, variant)) return rc;
   }
   // The call's first step is launched plainly, and the ones after it may overlap the kernel before them: that is
