@@ -132,12 +132,25 @@ inline bool pairs_eligible(const StepPlan& p) {
 }
 
 // Whether a 16-bit lattice that the span pipeline would take (variant 9) steps by the pair kernel
-// (variant 4): where nodes on a face are no operator's, they gather all values from global memory in the span
-// kernel's consumers and stall its tiles.  Measured (us a step, spans / pairs): Couette 100 x 90 x 110 44 / 30,
-// 130 x 97 x 113 82 / 42, 181 x 150 x 170 311 / 111; closed box 181 x 150 x 170 113 / 134.  MRT only where the
-// pair form runs (even z-planes), so that the stored bits stay the pair form's.
+// (variant 4; planes of odd size by the one-node kernel): nodes on faces that are no operator's gather all
+// values from global memory in the span kernel's consumers and stall its tiles.  On an open x face (periodic,
+// or bounced without an operator) they lie in every row, so every tile stalls; on open y and z faces they lie
+// together, and the pair kernel wins only where they are many.  Measured (us a step, BGK, pairs or one-node /
+// spans): x open: 181 x 150 x 170 105 / 242, 255 x 201 x 130 175 / 259.  x closed, open nodes in per cent:
+// 0 in 181 x 150 x 170 127 / 103; 0.1 in 37 x 37 x 2000 142 / 103; 1.2 in 181 x 150 x 170 133 / 123; 1.7 in
+// 140 x 109 x 120 65 / 65; 2.5 in 181 x 150 x 170 131 / 120; 3.0 in 150 x 131 x 140 92 / 99; 3.1 in 182 x 131 x 130
+// 95 / 89; 3.8 in 130 x 97 x 113 52 / 61; 5.4 in 37 x 37 x 2000 138 / 166.  Odd planes: 2.5 in 255 x 201 x 130
+// 199 / 145, 3.1 in 181 x 131 x 130 103 / 90, 4.0 in 101 x 91 x 111 41 / 43.  MRT only where the pair form runs
+// (even z-planes), so that the stored bits stay the pair form's.
 inline bool spans_avoided(const StepPlan& p) {
-  return p.face_mask != 0x3f && (p.collision == 0 || pairs_eligible(p));
+  const bool pairs = pairs_eligible(p);
+  if (p.collision != 0 && !pairs) return false;
+  if ((p.face_mask & 3) != 3) return true;
+  const int n[3] = {p.nx, p.ny, p.nz};
+  double open = 0.0;
+  for (int f = 2; f < 6; f++)
+    if (!(p.face_mask >> f & 1)) open += 1.0 / n[f / 2];
+  return open > (pairs ? 0.028 : 0.035);
 }
 
 // Whether a single-lattice launch of step variant `variant` (not the prologue) is followed by the
