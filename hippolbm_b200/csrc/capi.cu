@@ -477,14 +477,19 @@ cudaError_t outlet_passes(int prec, const StepPlan& p, void* fin, const int8_t* 
 
 // Whether a lattice steps in the resident kernel (lbm_step_resident.cuh): a plan it takes, no variant asked
 // for by hlbm_tune, and one node per thread of the GPU or, in the 16-bit tiers, both population buffers
-// within 50 MB.  Measured (us a step, resident against one launch a step): FP64 31^3 3.5 / 5.1, 48^3
-// 7.9 / 6.2; FP32 31^3 2.9 / 5.3, 48^3 6.2 / 6.2; FP16 31^3 3.8 / 15.2, 57 x 43 x 61 8.4 / 15.0, 80^3 (39 MB)
-// 18.1 / 16.9 couette and 18.0 / 34.6 cavity, 96^3 (67 MB) 29.8 / 21.9.  16-bit MRT keeps its step kernels:
-// there the node-pair form of every kernel has to round alike.
+// within 50 MB, or 24 MB where one launch a step needs no fix-up behind it.  Measured (us a step, resident
+// against one launch a step): FP64 31^3 3.7 / 4.8, 41^3 4.7 / 6.0; FP32 31^3 3.0 / 6.2; FP16 31^3 3.5 / 8.0,
+// 57 x 43 x 61 8.2 / 15.0.  FP16 with a fix-up: couette 64^3 10.0 / 14.0, 80^3 17.9 / 20.0, 88^3 (49 MB)
+// 20.8 / 24.7, cavity 80^3 18.3 / 24.6.  Without (periodic in x, y and z): 60^3 9.3 / 9.7, 64^3 (19 MB) 9.9 /
+// 12.3, 70^3 (25 MB) 13.2 / 12.0, 80^3 17.9 / 14.9.  16-bit MRT keeps its step kernels: there the node-pair
+// form of every kernel has to round alike.
 bool resident_applies(const hlbm_ctx* c) {
+  const StepPlan& p = c->plan;
   const bool half = elem_size(c->precision) == 2;
-  if (c->variant_forced || !resident_plan(c->plan) || (half && c->collision == 1)) return false;
-  return c->ncell <= int64_t(c->sms) * RES_THREADS || (half && 2 * int64_t(Q) * c->ncell * 2 <= int64_t(50) << 20);
+  if (c->variant_forced || !resident_plan(p) || (half && c->collision == 1)) return false;
+  const bool fixup = p.face_mask != 0 || (p.walls && p.wall_flags);
+  const int64_t limit = int64_t(fixup ? 50 : 24) << 20;
+  return c->ncell <= int64_t(c->sms) * RES_THREADS || (half && 2 * int64_t(Q) * c->ncell * 2 <= limit);
 }
 
 cudaError_t launch_resident_tier(int precision, const ResidentArgs& a, int walls, cudaStream_t s) {

@@ -206,7 +206,8 @@ int hlbm_info(hlbm_ctx* ctx, int64_t info[8]);
  * one node per thread.  A context starts at its tier's default (hlbm_autotune's pick on 512^3 Couette:
  * FP64 4, FP32 1, FP16 / BF16 9; 4 instead of 9 where rows are ragged and an x face, or many nodes on other
  * faces, are no boundary operator's) until hlbm_tune or hlbm_autotune chooses.  Until hlbm_tune chooses, hlbm_step advances
- * lattices that fit the GPU at one node per thread, and 16-bit BGK lattices of up to 50 MB, by many steps
+ * lattices that fit the GPU at one node per thread, and 16-bit BGK lattices of up to 50 MB (24 MB without
+ * boundary operators), by many steps
  * a launch of about a millisecond (not while the context's stream is being captured); such launches of
  * lattices on different streams run side by side up to 64 k nodes together (on 148 SMs), and one after
  * another beyond.  Variants 6, 7: persistent kernel fed by bulk asynchronous copies of whole rows

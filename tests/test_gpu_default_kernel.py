@@ -1,5 +1,5 @@
 """A 16-bit lattice starts with a kernel that is not much slower than the better of the pair kernel and the
-pipelines, whichever of its axes are periodic (rounds alternate, the fastest counts)."""
+pipelines, small or large and whichever of its axes are periodic (rounds alternate, the fastest counts)."""
 import time
 
 import pytest
@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 SPANS = [((255, 201, 130), (False, False, True)), ((255, 201, 130), (False, True, True)),
          ((181, 150, 170), (False, True, False)), ((181, 150, 170), (True, True, False)),
-         ((37, 37, 2000), (False, True, False)), ((37, 37, 2000), (False, False, True))]
+         ((37, 37, 2000), (False, True, False)), ((37, 37, 2000), (False, False, True)),
+         ((80, 80, 80), (True, True, True)), ((64, 64, 64), (True, True, True)), ((80, 80, 80), (True, True, False))]
 
 
 def box(nodes, periodic):

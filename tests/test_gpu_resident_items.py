@@ -36,7 +36,8 @@ def cases(kind):
                 box((61, 51, 41), (False, True, False),
                     start_iteration=[Op("set_distribution", {"value": 1.01, "bounds": [[3.0, 4.0, 5.0], [9.0, 9.0, 9.0]]})]),
                 box((61, 51, 41), (False, True, False), obstacles=ball)]
-    return [box(kind, axes, double_couette={"U": [0.03, 0.02, 0.0], "dimension": "Z"}) for axes in AXES]
+    # a lattice without boundary operators is stepped launch by launch from 24 MB on
+    return [box(kind, axes, double_couette={"U": [0.03, 0.02, 0.0], "dimension": "Z"}) for axes in AXES if not (all(axes) and np.prod(kind) * 76 > 24 << 20)]
 
 
 @pytest.mark.parametrize("precision", ["f16", "bf16"])
