@@ -1203,17 +1203,21 @@ int hlbm_get_populations(hlbm_ctx* c, double* out) {
   if (elem_size(c->precision) == 8) {
     HLBM_CK(g_host_copy.copy_rows(out, s, size_t(c->stride) * 8, n * 8, Q, c->stream));
   } else {
-    // several directions at a time, decoded side by side: about 64 MB, at least one; one where memory is short
+    // several directions at a time, decoded side by side in about 64 MB; large lattices, and where memory is
+    // short, one direction in the plane that hlbm_put_populations uses
     size_t group = std::min<size_t>(Q, std::max<size_t>(1, (size_t(64) << 20) / (n * 8)));
-    double* tmp = nullptr;
-    if (pool_alloc((void**)&tmp, group * n * 8, c->device, c->stream) != cudaSuccess) {
+    double* several = nullptr;
+    if (group > 1 && pool_alloc((void**)&several, group * n * 8, c->device, c->stream) != cudaSuccess) {
       cudaGetLastError();
+      several = nullptr;
       group = 1;
-      if (pool_alloc((void**)&tmp, n * 8, c->device, c->stream) != cudaSuccess) {
-        cudaGetLastError();
-        return fail(HLBM_ENOMEM, "hlbm_get_populations: no memory");
-      }
     }
+    if (group == 1 && !c->plane_tmp && pool_alloc((void**)&c->plane_tmp, n * 8, c->device, c->stream) != cudaSuccess) {
+      cudaGetLastError();
+      c->plane_tmp = nullptr;
+      return fail(HLBM_ENOMEM, "hlbm_get_populations: no memory");
+    }
+    double* const tmp = several ? several : c->plane_tmp;
     StepPlan p;
     base_plan(c, p);
     cudaError_t e = cudaSuccess;
@@ -1225,7 +1229,7 @@ int hlbm_get_populations(hlbm_ctx* c, double* out) {
       }
       if (e == cudaSuccess) e = g_host_copy.copy(out + i * n, tmp, k * n * 8, c->stream);
     }
-    pool_free(tmp, c->stream);
+    pool_free(several, c->stream);
     if (e != cudaSuccess) return fail(HLBM_ECUDA, std::string("hlbm_get_populations: ") + cudaGetErrorString(e));
   }
   HLBM_CK(cudaStreamSynchronize(c->stream));
