@@ -407,13 +407,18 @@ __device__ __forceinline__ void bgk(R (&v)[Q], const StepPlan& p) {
     static_assert(sizeof(R) == 8, "the other tiers collide by bgk_v");
     const R u_squ = __fma_rn(uz, uz, __fma_rn(uy, uy, __dmul_rn(ux, ux)));
     const R inv_tau = R(p.inv_tau);
-    Unroll<0, Q>::run([&]<int I>() {
+    const auto relax = [&]<int I>(R poly) {
       constexpr R w = weight<R, I>();
-      const R eu = edot<I, R>(ux, uy, uz);
-      const R poly = __fma_rn(R(-1.5), u_squ, __fma_rn(__dmul_rn(R(4.5), eu), eu, __fma_rn(R(3.), eu, R(1.))));
       R d = __dmul_rn(__fma_rn(__dmul_rn(w, rho), poly, -v[I]), inv_tau);
       if (force) d = __fma_rn(__dmul_rn(__dmul_rn(R(3.), rho), w), edot<I, R>(Fx, Fy, Fz), d);
       v[I] = __dadd_rn(v[I], d);
+    };
+    relax.template operator()<0>(__fma_rn(R(-1.5), u_squ, R(1.)));
+    Unroll<1, 10>::run([&]<int P>() {  // opposite directions: e.u changes sign, its square term stays
+      constexpr int I = 2 * P - 1;
+      const R eu = edot<I, R>(ux, uy, uz), eu45 = __dmul_rn(R(4.5), eu);
+      relax.template operator()<I>(__fma_rn(R(-1.5), u_squ, __fma_rn(eu45, eu, __fma_rn(R(3.), eu, R(1.)))));
+      relax.template operator()<I + 1>(__fma_rn(R(-1.5), u_squ, __fma_rn(eu45, eu, __fma_rn(R(-3.), eu, R(1.)))));
     });
   }
 }
