@@ -659,14 +659,12 @@ extern "C" {
 const char* hlbm_last_error(void) { return g_err.c_str(); }
 const char* hlbm_version(void) { return "hippolbm-b200 0.1.0 (sm_100a)"; }
 
-// Default step-kernel variant of a tier and collision: hlbm_autotune's pick on 512^3 Couette on a
-// B200.  FP64: one node per thread at >= 3 blocks/SM (4); FP32: 16-byte vectors at one block/SM
-// (1); FP16 / BF16: the row pipeline at two CTAs/SM (8) for BGK, one CTA/SM (9) for MRT (lattices
-// the row pipeline does not take run variant 5).
-static int default_variant(int precision, int collision) {
+// Default step-kernel variant of a tier: hlbm_autotune's pick on 512^3 Couette on a B200.  FP64: one node
+// per thread at >= 3 blocks/SM (4); FP32: 16-byte vectors at one block/SM (1); FP16 / BF16: the row
+// pipeline at one CTA/SM (9; the span pipeline on ragged rows, or variant 4 there by spans_avoided).
+static int default_variant(int precision) {
   if (precision == HLBM_F64 || precision == HLBM_F64_STRICT) return 4;
   if (precision == HLBM_F32) return 1;
-  (void)collision;
   return 9;
 }
 
@@ -699,7 +697,7 @@ int hlbm_domain(const int32_t cell_dims[3], const double bmin[3], const double b
   c->ncell = int64_t(n[0]) * n[1] * n[2];
   c->stride = (c->ncell + 127) / 128 * 128;
   if (precision == HLBM_F16) c->scale = 1024.0;
-  c->variant = default_variant(precision, 0);
+  c->variant = default_variant(precision);
   mrt_reference(c->mrt);
   auto cleanup = [&](int rc) {
     hlbm_destroy(c);
@@ -834,7 +832,7 @@ int hlbm_collision(hlbm_ctx* c, int32_t kind, const double* rates8) {
   StepPlan old_plan;
   base_plan(c, old_plan);
   c->collision = kind;
-  if (!c->variant_tuned) c->variant = default_variant(c->precision, kind);
+  if (!c->variant_tuned) c->variant = default_variant(c->precision);
   if (rates8)
     std::memcpy(c->mrt, rates8, sizeof(c->mrt));
   else

@@ -97,9 +97,8 @@ struct StepPlan {
   SetBox sets[MAX_SETS];
 };
 
-// Whether the kernels that update node pairs in packed FP32 (the vectorised kernel of the 4- and
-// 2-byte tiers, the 16-bit pair kernel, the row and span pipelines) take a plan: no start_iteration
-// boxes, and wall nodes only where wall_bounce_back makes their populations scratch (a pair collides
+// Whether the kernels that take several nodes at a time (the vectorised kernel of the 4- and 2-byte
+// tiers, the 16-bit pair kernel, the row and span pipelines) take a plan: no start_iteration boxes, and wall nodes only where wall_bounce_back makes their populations scratch (a pair collides
 // both lanes).  Other plans run the one-node kernel, and so does 16-bit MRT with a body force, whose
 // pair form may round differently.  (With a body force a 96^3 FP16 lattice steps in 30 us by the one-node
 // kernel, 22 by the row pipeline.)
@@ -119,7 +118,7 @@ inline constexpr int vec_npt_bytes(int bytes, int minb) {
 }
 inline constexpr int variant_minb(int variant) { return variant / 2 + 1; }
 inline bool vec_eligible_bytes(const StepPlan& p, int walls, int bytes, int variant) {
-  (void)walls;  // wall obstacles: the wall fix-up pass follows the vectorised kernel
+  (void)walls;  // wall obstacles: the fix-up follows the vectorised kernel
   const int npt = vec_npt_bytes(bytes, variant_minb(variant));
   return p.nx % npt == 0 && p.nx / npt >= 32 && p.ncell <= int64_t(0xffffffffu) && pair_kernels_apply(p, bytes);
 }
@@ -153,9 +152,9 @@ inline bool spans_avoided(const StepPlan& p) {
   return open > (pairs ? 0.028 : 0.035);
 }
 
-// Whether a single-lattice launch of step variant `variant` (not the prologue) is followed by the
-// face pass: the vectorised kernel always, the one-node kernel for the 4- and 2-byte tiers; the
-// pipelined kernel (variants 6, 7) applies the operators inline.
+// Whether a read-out by the kernel of step variant `variant` is followed by the face pass: the vectorised
+// kernel always, the one-node kernel for the 4- and 2-byte tiers; the pipelined kernel (variants 6, 7)
+// applies the operators inline.
 inline bool face_pass_runs(const StepPlan& p, int walls, int variant, bool prologue, int bytes) {
   if (variant >= 6 || prologue || p.face_mask == 0) return false;
   return (variant % 2 == 1 && vec_eligible_bytes(p, walls, bytes, variant)) || bytes < 8;

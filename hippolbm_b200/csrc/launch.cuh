@@ -61,8 +61,8 @@ cudaError_t launch_fixup(const S* fi, S* fo, const int8_t* flags, const StepPlan
   return launch_kernel(k_fixup<S, R, STRICT, WALLS, 1>, grid, dim3(FIX_THREADS), 0, p, s, early, fi, fo, flags, p, g);
 }
 
-// The face pass after a step kernel that left the boundary operators out: the nodes of the faces
-// in p.face_mask, recomputed whole by the one-node step.
+// The nodes of the faces in p.face_mask after a kernel that left the boundary operators out, recomputed whole by
+// the one-node step: the fix-up of a fused step, the face pass of a read-out.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS>
 cudaError_t launch_faces(const S* fi, S* fo, const int8_t* flags, const StepPlan& p, cudaStream_t s) {
   const int faces = p.face_mask;
@@ -256,8 +256,7 @@ cudaError_t launch_tiles(const TmaArgs& a, int walls, int variant, cudaStream_t 
 }
 
 // The row pipeline (lbm_step_rows.cuh) for one lattice: variant 8 = two CTAs per SM, variant 9 =
-// one CTA per SM with deeper staging; the face pass and (with wall obstacles) the wall fix-up
-// follow.  Returns cudaErrorNotSupported when the lattice or the mode cannot take it.
+// one CTA per SM with deeper staging; the fix-up follows.  Returns cudaErrorNotSupported when the lattice or the mode cannot take it.
 constexpr int rows_stage_count(int warps, int ctas_per_sm) {
   const size_t budget = size_t(227 * 1024) / size_t(ctas_per_sm) - 1024;
   const size_t fit = (budget - 128) / rows_stage_bytes(warps);

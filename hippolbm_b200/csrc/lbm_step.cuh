@@ -1071,7 +1071,7 @@ __device__ __forceinline__ void node_update(R (&v)[Q], const S* fin, int64_t idx
 // pair kernels take lattices whose non-fluid nodes are walls under wall_bounce_back
 // (pair_kernels_apply): a wall node's populations are scratch that no fluid node reads, so it
 // collides with its partner and then stores the read-out value of a wall.  No boundary operators
-// (a face pass applies them) and no start_iteration boxes (plans with boxes run the one-node
+// (the fix-up or a read-out's face pass applies them) and no start_iteration boxes (plans with boxes run the one-node
 // kernel).  Each fluid lane gets exactly the arithmetic node_update gives its node.
 template <typename S, int MODE, int COLL>
 __device__ __forceinline__ void pair_update(float2 (&v)[Q], const StepPlan& p, int8_t fa, int8_t fb) {
@@ -1189,8 +1189,8 @@ __device__ __forceinline__ void node_step(const S* fin, S* __restrict__ fout,
   store_node<S, R, MODE>(v, p, launch_seed<S>(p), idx, [&]<int I>(S s) { fout[I * p.stride + idx] = s; });
 }
 
-// Storage types whose one-node step kernel leaves the boundary operators to the face pass (k_faces):
-// the 4- and 2-byte tiers, whose kernels are bound by instruction issue, so the operator code
+// Storage types whose one-node step kernel leaves the boundary operators to the fix-up (k_fixup) or, in a
+// read-out, the face pass (k_faces): the 4- and 2-byte tiers, whose kernels are bound by instruction issue, so the operator code
 // costs there.  FP64 applies them inline: its kernel runs at the copy bandwidth either way.
 template <typename S>
 constexpr bool face_pass_tier() {
@@ -1223,7 +1223,7 @@ __global__ void __launch_bounds__(256, MINB) k_step(const S* fin, S* __restrict_
     z = blockIdx.z;
     if (x >= p.nx || y >= p.ny) return;
   }
-  // the face pass computes the operator faces after this kernel (not after a prologue): whole
+  // the operator faces are computed after this kernel (not after a prologue): whole
   // z-face planes are skipped (a uniform test per block), other face nodes are computed twice
   if (face_pass_tier<S>() && MODE != MODE_PROLOGUE && on_op_z_face(p, z)) return;
   node_step<S, R, STRICT, MODE, WALLS, COLL, !face_pass_tier<S>()>(fin, fout, flags, p, x, y, z);
@@ -1232,7 +1232,7 @@ __global__ void __launch_bounds__(256, MINB) k_step(const S* fin, S* __restrict_
 // The one-node step of the 16-bit tiers, two consecutive nodes of a z-plane per thread: each
 // direction's two results convert into one packed word and one 32-bit store (plane sizes even, so
 // every pair starts on a 4-byte boundary; below 2^24 nodes, for the index arithmetic of `linear`).
-// Boundary operators are left to the face pass.  A wall node of a pair stores the read-out value
+// Boundary operators are left to the fix-up or the face pass.  A wall node of a pair stores the read-out value
 // of a wall (population 0); the one-node kernel leaves that slot untouched, and no fluid node
 // reads it either way.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL, int MINB>
@@ -1259,7 +1259,7 @@ __global__ void __launch_bounds__(256, MINB) k_step_pairs(const S* fin, S* __res
     xb = 0;
     yb++;
   }
-  // a z-face plane: the face pass computes it after this kernel
+  // a z-face plane is computed after this kernel
   if (MODE != MODE_PROLOGUE && on_op_z_face(p, z)) return;
   const int64_t idx = int64_t(z) * plane + i;
   const int8_t fa = flags[idx], fb = flags[idx + 1];
@@ -1278,9 +1278,9 @@ __global__ void __launch_bounds__(256, MINB) k_step_pairs(const S* fin, S* __res
   pack_pair<S>(v, sr, h, h2, [&]<int I>(uint32_t w) { *reinterpret_cast<uint32_t*>(fout + I * p.stride + idx) = w; });
 }
 
-// The face pass of the vectorised kernels: the nodes of the faces in `faces` (bit F = face F),
-// each stepped whole by node_step, after the vectorised kernel stepped them without boundary
-// operators.  Both read only fin, so the pass overwrites those nodes' outputs with the complete
+// The face pass of a read-out: the nodes of the faces in `faces` (bit F = face F),
+// each streamed whole by node_step, after a kernel that left their boundary operators out.
+// Both read only fin, so the pass overwrites those nodes' outputs with the complete
 // update.  blockIdx.y is the face; nodes on two faces are computed twice, to the same bits.
 template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL>
 __global__ void __launch_bounds__(256) k_faces(const S* fin, S* __restrict__ fout,
@@ -1318,9 +1318,10 @@ __global__ void __launch_bounds__(256) k_faces(const S* fin, S* __restrict__ fou
 
 // The fix-up after a fused step: the nodes on the operator faces, and (list) those next to walls after
 // the kernels that pull without testing for walls, each once and whole by the one-node step.  It
-// reads only fin, as the step kernel does, and overwrites that kernel's results.  One launch, 128 threads a block (more blocks for the few nodes
-// there are, and one fits beside a pipeline CTA).  The face pass and the scan of the near-wall map that it
-// replaces took 23 + 31 us after a 45 us span kernel on a 150 x 120 x 131 sphere.
+// reads only fin, as the step kernel does, and overwrites that kernel's results.  One launch, 128 threads a
+// block: more blocks for the few nodes there are.  Bound by the latency of one round of loads and a collision,
+// and by the sectors of the x faces.  The face pass and the scan of the near-wall map that it replaces took
+// 23 + 31 us after a 45 us span kernel on a 150 x 120 x 131 sphere; it takes 30.
 struct FixGeometry {
   uint32_t nx_items = 0, ny_items = 0, nz_items = 0;  // nodes of the x, y and z faces
   uint32_t total = 0;

@@ -16,8 +16,8 @@
 // global memory with one 8- or 16-byte store per direction.  STAGES tiles are in flight while the
 // consumers compute, so memory latency is off the consumers' path and few registers hold data.
 //
-// Like the vectorised kernel it applies no boundary operator (the face pass follows) and no wall
-// test (the wall fix-up follows on lattices with wall obstacles), and takes fused steps only.
+// Like the vectorised kernel it applies no boundary operator and no wall test (the fix-up follows), and
+// takes fused steps only.
 // Copies are plain (non-multicast) bulk loads of this GPU's own memory; every wait is bounded.
 #pragma once
 #include <cuda_runtime.h>
@@ -70,8 +70,10 @@ inline RowsGeometry rows_geometry(const StepPlan& p, int warps) {
 }
 
 // Whether variant 9 takes 15 consumer warps, a tile of 1,920 nodes, instead of 12: where whole rows fill
-// its tile at least a tenth better.  Measured (us a step, 12 / 15 warps): nx = 320, 5/6 of the small tile and
-// all of the wide one, MRT 596 / 538 at 320^3; nx = 384, both full, BGK 246 / 255 and MRT 317 / 308 at
+// its tile at least a tenth better (nx = 272, 320, 528 to 640, 784 to 960).  Measured (us a step, 12 / 15 warps,
+// lattices of 24 M nodes, BGK and MRT): nx = 272 372 / 338 and 465 / 409; 320, 5/6 of the small tile and all of
+// the wide one, 362 / 338 and 445 / 404; 528 475 / 395 and 578 / 473; 640 368 / 332 and 455 / 393; 784 509 / 384
+// and 622 / 456; 960 439 / 345 and 535 / 397.  Not taken: nx = 384, both full, BGK 246 / 255 and MRT 317 / 308 at
 // 384^2 x 128; nx = 512, full and 4/5, BGK 441 / 482.
 inline bool rows_wide(const StepPlan& p) {
   const auto fill = [&](int warps) {

@@ -14,11 +14,10 @@
 //
 // A group of four nodes whose sources all lie inside the lattice (no node on a face, all in one
 // row) reads only the stage.  In the other groups the nodes off the faces still read the stage;
-// a face node either lies on a face the face pass recomputes (left for it) or pulls all its values
+// a face node either lies on a face the fix-up recomputes (left for it) or pulls all its values
 // from global memory with the one-node kernel's gather (periodic wrap, on-node bounce-back).
-// Like the row pipeline it applies no boundary operator (the face pass follows), no wall test (the
-// wall fix-up follows on lattices with wall obstacles), and takes fused steps of the 16-bit tiers
-// only; the node pairs (n, n + 1), n even, and their random bits are those of every other kernel,
+// Like the row pipeline it applies no boundary operator and no wall test (the fix-up follows), and takes
+// fused steps of the 16-bit tiers only; the node pairs (n, n + 1), n even, and their random bits are those of every other kernel,
 // so its results equal theirs bit for bit.  Copies are plain (non-multicast) bulk loads of this
 // GPU's own memory; every wait is bounded.
 #pragma once
@@ -85,7 +84,7 @@ inline int spans_stages(const SpansGeometry& g, int ctas_per_sm) {
   return fit >= 4 ? 4 : int(fit);
 }
 
-// Whether node (x, y, z) lies on a face whose nodes the face pass recomputes.
+// Whether node (x, y, z) lies on a face whose nodes the fix-up recomputes.
 __device__ __forceinline__ bool on_pass_face(const StepPlan& p, int x, int y, int z) {
   const int m = p.face_mask;
   return ((m & 1) && x == 0) || ((m & 2) && x == p.nx - 1) || ((m & 4) && y == 0) || ((m & 8) && y == p.ny - 1) ||
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
     if (lane == 0) mbar_arrive(&empty[s]);
     if (!active) continue;
     if (!interior) {
-      // a group at a face or across a row end: face nodes the face pass recomputes keep the staged
+      // a group at a face or across a row end: face nodes the fix-up recomputes keep the staged
       // (meaningless) values; other face nodes gather theirs from global memory
       int live = 0;
       Unroll<0, ROWS_NODES_PER_THREAD>::run([&]<int J>() {
@@ -224,7 +223,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
           w = (J & 1) ? (w & 0x0000ffffu) | (b << 16) : (w & 0xffff0000u) | b;
         });
       });
-      if (live == 0) continue;  // every node is left to the face pass or lies past the lattice
+      if (live == 0) continue;  // every node is left to the fix-up or lies past the lattice
     }
     Unroll<0, 2>::run([&]<int J>() {
       const int8_t fa = int8_t(fl4 >> (16 * J)), fb = int8_t(fl4 >> (16 * J + 8));

@@ -1,7 +1,6 @@
 // lbm_step_vec.cuh -- the fused step with NPT consecutive x-nodes per thread.
 //
-// Same step as k_step (lbm_step.cuh), for lattices without wall obstacles: every direction
-// plane is read and written as one aligned vector per thread (16 bytes: double2, float4, 8 packed
+// Same step as k_step (lbm_step.cuh), without its wall test: every direction plane is read and written as one aligned vector per thread (16 bytes: double2, float4, 8 packed
 // FP16/BF16 values; or 8 bytes at the highest occupancy target: float2, 4 packed 16-bit values),
 // which multiplies the bytes each thread keeps in flight by NPT.  All loads
 // of a thread are issued before the first shuffle consumes one, so they overlap.
@@ -9,10 +8,11 @@
 // it comes from a warp shuffle, and lanes at a warp edge fetch it with one scalar load (the
 // element of the previous/next warp, or the periodic image / on-node bounce-back at a row
 // end).  Warps never straddle rows: the x extent of a block is a multiple of 32 threads.
-// The kernel applies no boundary operator: the launcher follows it with the face pass (k_faces),
-// which recomputes the nodes of the faces those operators touch, so the per-node code here stays
-// small.  The 4- and 2-byte tiers update the nodes in pairs, the two lanes of packed FP32
-// arithmetic (lanes.cuh); the 16-bit tiers convert each pair into packed words.
+// The kernel applies no boundary operator: the launcher follows it with the fix-up (k_fixup; in a
+// read-out k_faces and k_wall_fixup), which recomputes the nodes of the faces those operators touch
+// and those next to walls, so the per-node code here stays small.  16-bit MRT collides node pairs, the two
+// lanes of packed FP32 arithmetic (lanes.cuh), everything else one node at a time; the 16-bit tiers
+// convert each pair's results into packed words.
 #pragma once
 #include <type_traits>
 
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256, MINB) k_step_vec(const __grid_constant__ 
   const int lane = threadIdx.x & 31;
   const int x0 = tx < nvec ? tx * NPT : 0;
   const int yy = y < p.ny ? y : p.ny - 1;
-  // a row on an operator face (y or z): the face pass computes all of it after this kernel.  The
+  // a row on an operator face (y or z): all of it is computed after this kernel.  The
   // condition is uniform over the warp (one row), so no shuffle partner is missing.
   if (MODE != MODE_PROLOGUE && (p.face_mask >> 2) != 0 &&
       (((p.face_mask >> 2) & 1) && yy == 0 || ((p.face_mask >> 3) & 1) && yy == p.ny - 1 ||

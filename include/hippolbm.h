@@ -201,16 +201,15 @@ int hlbm_info(hlbm_ctx* ctx, int64_t info[8]);
  * 5 for the FP32 and 16-bit tiers, 16 bytes always for FP64; used when nx splits into >= 32
  * vectors, else the first kernel runs; with wall obstacles a fix-up launch re-steps the nodes next
  * to walls); variant / 2 = 0, 1, 2 targets at least 1, 2 or 3 blocks of 256 threads per SM.
- * The FP32 and 16-bit tiers update node pairs in packed FP32 where a plan has no start_iteration
- * boxes, no wall nodes outside wall_bounce_back and, with 16-bit MRT, no body force; other plans run
- * one node per thread.  A context starts at its tier's default (hlbm_autotune's pick on 512^3 Couette:
- * FP64 4, FP32 1, FP16 / BF16 9; 4 instead of 9 where rows are ragged and an x face, or many nodes on other
- * faces, are no boundary operator's) until hlbm_tune or hlbm_autotune chooses.  Until hlbm_tune chooses, hlbm_step advances
- * lattices that fit the GPU at one node per thread, and 16-bit BGK lattices of up to 50 MB (24 MB without
- * boundary operators), by many steps
- * a launch of about a millisecond (not while the context's stream is being captured); such launches of
- * lattices on different streams run side by side up to 64 k nodes together (on 148 SMs), and one after
- * another beyond.  Variants 6, 7: persistent kernel fed by bulk asynchronous copies of whole rows
+ * The FP32 and 16-bit tiers take several nodes at a time (16-bit ones as pairs in packed FP32) where a
+ * plan has no start_iteration boxes, no wall nodes outside wall_bounce_back and, with 16-bit MRT, no
+ * body force; other plans run one node per thread.  A context starts at its tier's default (hlbm_autotune's pick on 512^3 Couette:
+ * FP64 4, FP32 1, FP16 / BF16 9; 4 instead of 9 where rows are ragged and an x face, or many nodes on
+ * other faces, are no boundary operator's) until hlbm_tune or hlbm_autotune chooses.  Until hlbm_tune
+ * chooses, hlbm_step advances lattices that fit the GPU at one node per thread, and 16-bit BGK lattices
+ * of up to 50 MB (24 MB without boundary operators and walls), by many steps a launch of about a
+ * millisecond (not while the context's stream is being captured); such launches of lattices on different
+ * streams run side by side up to some 64 k nodes together (on 148 SMs), and one after another beyond.  Variants 6, 7: persistent kernel fed by bulk asynchronous copies of whole rows
  * into shared-memory stages (256 or 512 threads per CTA; needs nx * bytes per population to be a
  * multiple of 16; otherwise variant 4 runs).  hlbm_autotune times `reps` fused launches of every
  * variant on this lattice (from the current populations into the idle buffer, so the state does
