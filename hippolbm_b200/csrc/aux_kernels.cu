@@ -426,24 +426,29 @@ cudaError_t launch_rasterize(int8_t* flags, const StepPlan& p, const int lo[3], 
 // near[idx] = 2 for a wall node, else 1 when a direction of node idx pulls from a wall node (the pull the step kernels
 // replace by on-node bounce-back under wall_bounce_back), with the gather's periodic wrap; pulls
 // from outside a non-periodic face bounce anyway and are not counted.
+// Inner nodes take one constant offset per direction and all loads at once; with the general loop for every
+// node, 320^3 took 1.0 ms, 0.34 now.
 __global__ void k_near_wall(const int8_t* __restrict__ flags, int8_t* __restrict__ near, int nx, int ny, int nz,
                             int px, int py, int pz) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
   if (x >= nx) return;
-  int8_t any = 0;
-  for (int dz = -1; dz <= 1; dz++)
-    for (int dy = -1; dy <= 1; dy++)
-      for (int dx = -1; dx <= 1; dx++) {
-        const int m = (dx != 0) + (dy != 0) + (dz != 0);
-        if (m == 0 || m == 3) continue;  // D3Q19: the 6 axis and 12 edge neighbours
-        int sx = x + dx, sy = y + dy, sz = z + dz;
-        if (sx < 0 || sx >= nx) { if (!px) continue; sx = sx < 0 ? sx + nx : sx - nx; }
-        if (sy < 0 || sy >= ny) { if (!py) continue; sy = sy < 0 ? sy + ny : sy - ny; }
-        if (sz < 0 || sz >= nz) { if (!pz) continue; sz = sz < 0 ? sz + nz : sz - nz; }
-        if (flags[(int64_t(sz) * ny + sy) * nx + sx] == FLAG_WALL) any = 1;
-      }
   const int64_t idx = (int64_t(z) * ny + y) * nx + x;
-  near[idx] = flags[idx] == FLAG_WALL ? 2 : any;
+  bool any = false;
+  if (x > 0 && x < nx - 1 && y > 0 && y < ny - 1 && z > 0 && z < nz - 1) {
+    const int64_t plane = int64_t(nx) * ny;
+    Unroll<1, Q>::run([&]<int I>() {
+      any |= flags[idx + D3Q19::ez[I] * plane + D3Q19::ey[I] * nx + D3Q19::ex[I]] == FLAG_WALL;
+    });
+  } else {
+    for (int i = 1; i < Q; i++) {
+      int sx = x + dir_ex(i), sy = y + dir_ey(i), sz = z + dir_ez(i);
+      if (sx < 0 || sx >= nx) { if (!px) continue; sx = sx < 0 ? sx + nx : sx - nx; }
+      if (sy < 0 || sy >= ny) { if (!py) continue; sy = sy < 0 ? sy + ny : sy - ny; }
+      if (sz < 0 || sz >= nz) { if (!pz) continue; sz = sz < 0 ? sz + nz : sz - nz; }
+      any |= flags[(int64_t(sz) * ny + sy) * nx + sx] == FLAG_WALL;
+    }
+  }
+  near[idx] = flags[idx] == FLAG_WALL ? 2 : (any ? 1 : 0);
 }
 
 // Counts the near-wall nodes or, with `list`, writes them down: one atomic per warp, so the nodes of

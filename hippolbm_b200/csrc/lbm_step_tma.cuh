@@ -59,8 +59,10 @@ constexpr uint64_t pack_component(const int* e) {
   for (int i = 0; i < Q; i++) v |= uint64_t(e[i] + 1) << (2 * i);
   return v;
 }
+constexpr uint64_t EX_PACKED = pack_component(D3Q19::ex);
 constexpr uint64_t EY_PACKED = pack_component(D3Q19::ey);
 constexpr uint64_t EZ_PACKED = pack_component(D3Q19::ez);
+__device__ __forceinline__ int dir_ex(int i) { return int((EX_PACKED >> (2 * i)) & 3u) - 1; }
 __device__ __forceinline__ int dir_ey(int i) { return int((EY_PACKED >> (2 * i)) & 3u) - 1; }
 __device__ __forceinline__ int dir_ez(int i) { return int((EZ_PACKED >> (2 * i)) & 3u) - 1; }
 __device__ __forceinline__ int dir_opp(int i) { return i == 0 ? 0 : ((i & 1) ? i + 1 : i - 1); }
