@@ -332,8 +332,18 @@ __global__ void __launch_bounds__(256) k_moments(const S* __restrict__ f, const 
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < ncell;
        idx += (int64_t)gridDim.x * blockDim.x) {
     if (flags[idx] < FLAG_FLUID) continue;
+    // FP64 and 16-bit values are loaded in the order of the source, before one is used: left to the
+    // compiler, a 320^3 FP16 lattice took 1.27 ms in one build and 0.56 in another (0.47 so).  FP32: 1.32 in order,
+    // 1.24 so
+    S raw[Q];
+    Unroll<0, Q>::run([&]<int I>() {
+      if constexpr (sizeof(S) == 4)
+        raw[I] = f[I * p.stride + idx];
+      else
+        raw[I] = ld_l2(f + I * p.stride + idx);
+    });
     double v[Q];
-    Unroll<0, Q>::run([&]<int I>() { v[I] = double(Codec<S, R>::template dec<I>(f[I * p.stride + idx], p)); });
+    Unroll<0, Q>::run([&]<int I>() { v[I] = double(Codec<S, R>::template dec<I>(raw[I], p)); });
     double rho = v[0];
     for (int i = 1; i < Q; i++) rho += v[i];
     acc[0] += rho;
