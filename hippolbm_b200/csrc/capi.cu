@@ -1058,7 +1058,10 @@ int hlbm_step(hlbm_ctx* c, int64_t nsteps) {
     nsteps--;
   }
   if (nsteps > 0 && !captured) {
-    if (resident_applies(c)) {
+    // One step that needs no fix-up launch is quicker as a plain launch: 31^3 FP64, ten calls of one step each,
+    // 90 us against 119 (FP32 with a fix-up 158 / 103; two steps a call FP64 170 / 147).
+    const bool fixup = elem_size(c->precision) < 8 && (c->plan.face_mask != 0 || walks_near_list(c, variant));
+    if ((nsteps > 1 || fixup) && resident_applies(c)) {
       int64_t done = 0;
       if (int rc = resident_steps(c, nsteps, done)) return rc;
       nsteps -= done;

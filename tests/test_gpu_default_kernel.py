@@ -40,3 +40,25 @@ def test_default_is_a_fast_kernel(nodes, periodic):
     for lat in lats:
         lat.close()
     assert best[0] <= 1.15 * min(best)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+def test_calls_of_one_step_are_quick(precision):
+    """A small lattice stepped one step a call, without a fix-up launch: no slower than its step kernel."""
+    from hippolbm_b200.lattice import Lattice
+
+    lats = [Lattice.from_case(box((31, 31, 31), (True, True, True)), precision) for _ in range(2)]
+    lats[1].tune(4)
+    best = [1e9] * 2
+    for _ in range(8):
+        for k, lat in enumerate(lats):
+            lat.step(2)
+            lat.sync()
+            t = time.perf_counter()
+            for _ in range(100):
+                lat.step(1)
+            lat.sync()
+            best[k] = min(best[k], time.perf_counter() - t)
+    for lat in lats:
+        lat.close()
+    assert best[0] <= 1.2 * best[1]
