@@ -601,16 +601,16 @@ bool vec_applies(const hlbm_ctx* c, int variant) {
   return vec_eligible_bytes(c->plan, c->plan.walls, int(elem_size(c->precision)), variant);
 }
 
-// {sum rho, min |u|, max |u|} of S_k into stats_dev, from the post-collision state in fin
-cudaError_t observe_state(hlbm_ctx* c, const void* fin) {
+// {sum rho, min |u|, max |u|} of S_k into stats_dev, from the post-collision state in fin; S_k into fout unless null
+cudaError_t observe_state(hlbm_ctx* c, const void* fin, void* fout) {
   const int blocks = stats_blocks(c->ncell);
   unsigned* done = c->group_dev;  // zero between launches, like the many-step launches' counter
   switch (c->precision) {
-    case HLBM_F64: return observe_f64(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
-    case HLBM_F64_STRICT: return observe_f64_strict(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
-    case HLBM_F32: return observe_f32(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
-    case HLBM_F16: return observe_f16(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
-    default: return observe_bf16(fin, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F64: return observe_f64(fin, fout, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F64_STRICT: return observe_f64_strict(fin, fout, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F32: return observe_f32(fin, fout, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    case HLBM_F16: return observe_f16(fin, fout, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
+    default: return observe_bf16(fin, fout, c->flags, c->plan, blocks, c->partials, done, c->stats_dev, c->stream);
   }
 }
 
@@ -1117,12 +1117,14 @@ int hlbm_macro_variables(hlbm_ctx* c, double* rho, double* u) {
 int hlbm_simulation_state(hlbm_ctx* c, double out[3]) {
   if (!c || !out) return fail(HLBM_EINVAL, "hlbm_simulation_state: NULL argument");
   if (int rc = set_device(c)) return rc;
-  if (c->phase == POSTCOL) {  // straight from the post-collision state; the idle buffer stays idle
+  bool stored = false;
+  if (c->phase == POSTCOL) {  // straight from the post-collision state
     if (int rc = build_plan(c)) return rc;
+    stored = observe_stores(c->plan);
     void* fin = c->f[c->cur];
     HLBM_CK(outlet_passes(c->precision, c->plan, fin, c->flags, c->stream, c->launches));
     c->launches++;
-    HLBM_CK(observe_state(c, fin));
+    HLBM_CK(observe_state(c, fin, stored ? c->f[1 - c->cur] : nullptr));
   } else {
     const void* s = c->phase == RAW ? c->f[c->cur] : c->f[1 - c->cur];
     StepPlan p;
@@ -1137,6 +1139,7 @@ int hlbm_simulation_state(hlbm_ctx* c, double out[3]) {
   HLBM_CK(cudaMemcpyAsync(h, c->stats_dev, 3 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   HLBM_CK(cudaStreamSynchronize(c->stream));
   if (e != 0) return check_device_error(c);
+  if (stored) c->phase = MATER;
   for (int k = 0; k < 3; k++) out[k] = h[k];
   return HLBM_OK;
 }

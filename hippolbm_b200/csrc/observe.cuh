@@ -7,6 +7,10 @@
 // operators of the read-out), rounds it as the read-out would store it, and takes its macro variables;
 // the last block to finish folds the partial sums.  Sums run in the order of k_macro_stats and
 // k_reduce_partials (aux_kernels.cu), without contraction, so the values are the same.
+//
+// STORE: the rounded state is stored as the read-out would store it, so that another read-out of the same
+// step finds it.  It costs a tenth to a fifth of the pass and saves one, which pays on large lattices:
+// observe_stores.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -23,9 +27,15 @@ __device__ __forceinline__ double readout_value(R v, const StepPlan& p) {
     return double(v);
 }
 
+// Whether simulation_state stores the state: lattices of a million nodes and more.  Measured (us, one step and
+// simulation_state / those and moments; before this kernel, without, with storing): FP64 31^3 57, 46, 44 /
+// 104, 92, 84; FP16 128^3 205, 167, 180 / 272, 291, 250; FP64 320^3 3873, 2843, 3209 / 5276, 5427, 4301; ten
+// steps and simulation_state FP64 31^3 122, 78, 82; 64 x 60 x 61 224, 172, 176.
+inline bool observe_stores(const StepPlan& p) { return p.ncell >= (int64_t(1) << 20); }
+
 // out: {sum rho, min |u|, max |u|}; done: blocks finished, zero between launches
-template <typename S, typename R, bool STRICT, bool WALLS>
-__global__ void __launch_bounds__(256) k_observe(const S* fin, const int8_t* __restrict__ flags,
+template <typename S, typename R, bool STRICT, bool WALLS, bool STORE>
+__global__ void __launch_bounds__(256) k_observe(const S* fin, S* __restrict__ fout, const int8_t* __restrict__ flags,
                                                  const __grid_constant__ StepPlan p, double* __restrict__ partials,
                                                  unsigned* __restrict__ done, double* __restrict__ out) {
   double s = 0.0, vmin = 1.79769313486231570815e+308, vmax = -1.79769313486231570815e+308;
@@ -33,7 +43,9 @@ __global__ void __launch_bounds__(256) k_observe(const S* fin, const int8_t* __r
   for (int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; idx < p.ncell; idx += int64_t(gridDim.x) * blockDim.x) {
     double rho = 0.0, ux = 0.0, uy = 0.0, uz = 0.0;
     const int8_t flag = flags[idx];
-    if (flag >= FLAG_FLUID) {
+    if (STORE && WALLS && flag == FLAG_WALL) {
+      Unroll<0, Q>::run([&]<int I>() { fout[I * p.stride + idx] = Codec<S, R>::template enc<I>(R(0), p); });
+    } else if (STORE || flag >= FLAG_FLUID) {
       const int z = int(idx / plane);
       const int64_t rem = idx - z * plane;
       const int y = int(rem / p.nx), x = int(rem - int64_t(y) * p.nx);
@@ -42,9 +54,12 @@ __global__ void __launch_bounds__(256) k_observe(const S* fin, const int8_t* __r
       R v[Q];
       Unroll<0, Q>::run([&]<int I>() { v[I] = load_value<S, R, I>(raw[I], p); });
       node_update<S, R, STRICT, MODE_FINISH, 2>(v, fin, idx, x, y, z, flag, p, true, on_op_face(p, x, y, z));
-      double d[Q];
-      Unroll<0, Q>::run([&]<int I>() { d[I] = readout_value<S, R, I>(v[I], p); });
-      macro<double, true>(d, rho, ux, uy, uz);
+      if constexpr (STORE) store_node<S, R, MODE_FINISH>(v, p, 0, idx, [&]<int I>(S s) { fout[I * p.stride + idx] = s; });
+      if (!STORE || flag >= FLAG_FLUID) {
+        double d[Q];
+        Unroll<0, Q>::run([&]<int I>() { d[I] = readout_value<S, R, I>(v[I], p); });
+        macro<double, true>(d, rho, ux, uy, uz);
+      }
     }
     s = __dadd_rn(s, rho);
     const double n = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz)));
@@ -110,20 +125,32 @@ __global__ void __launch_bounds__(256) k_observe(const S* fin, const int8_t* __r
   }
 }
 
-template <typename S, typename R, bool STRICT>
-cudaError_t launch_observe(const void* fin, const int8_t* flags, const StepPlan& p, int blocks, double* partials,
-                           unsigned* done, double* out, cudaStream_t s) {
-  if (p.walls)
-    k_observe<S, R, STRICT, true><<<blocks, 256, 0, s>>>(static_cast<const S*>(fin), flags, p, partials, done, out);
+template <typename S, typename R, bool STRICT, bool WALLS>
+void launch_observe_walls(const void* fin, void* fout, const int8_t* flags, const StepPlan& p, int blocks,
+                          double* partials, unsigned* done, double* out, cudaStream_t s) {
+  const S* fi = static_cast<const S*>(fin);
+  S* fo = static_cast<S*>(fout);
+  if (fo)
+    k_observe<S, R, STRICT, WALLS, true><<<blocks, 256, 0, s>>>(fi, fo, flags, p, partials, done, out);
   else
-    k_observe<S, R, STRICT, false><<<blocks, 256, 0, s>>>(static_cast<const S*>(fin), flags, p, partials, done, out);
+    k_observe<S, R, STRICT, WALLS, false><<<blocks, 256, 0, s>>>(fi, fo, flags, p, partials, done, out);
+}
+
+// fout: where the state is stored, or null
+template <typename S, typename R, bool STRICT>
+cudaError_t launch_observe(const void* fin, void* fout, const int8_t* flags, const StepPlan& p, int blocks,
+                           double* partials, unsigned* done, double* out, cudaStream_t s) {
+  if (p.walls)
+    launch_observe_walls<S, R, STRICT, true>(fin, fout, flags, p, blocks, partials, done, out, s);
+  else
+    launch_observe_walls<S, R, STRICT, false>(fin, fout, flags, p, blocks, partials, done, out, s);
   return cudaGetLastError();
 }
 
 // one entry per precision tier (defined in resident_*.cu)
 #define HLBM_OBSERVE_ENTRY(tier)                                                                                   \
-  cudaError_t observe_##tier(const void* fin, const int8_t* flags, const StepPlan& p, int blocks, double* partials, \
-                             unsigned* done, double* out, cudaStream_t s)
+  cudaError_t observe_##tier(const void* fin, void* fout, const int8_t* flags, const StepPlan& p, int blocks,      \
+                             double* partials, unsigned* done, double* out, cudaStream_t s)
 HLBM_OBSERVE_ENTRY(f64_strict);
 HLBM_OBSERVE_ENTRY(f64);
 HLBM_OBSERVE_ENTRY(f32);

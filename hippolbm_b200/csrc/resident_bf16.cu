@@ -8,6 +8,6 @@ cudaError_t resident_bf16(const ResidentArgs& a, int walls, cudaStream_t s) {
   return launch_resident<__nv_bfloat16, float, false>(a, walls, s);
 }
 HLBM_OBSERVE_ENTRY(bf16) {
-  return launch_observe<__nv_bfloat16, float, false>(fin, flags, p, blocks, partials, done, out, s);
+  return launch_observe<__nv_bfloat16, float, false>(fin, fout, flags, p, blocks, partials, done, out, s);
 }
 }  // namespace hlbm

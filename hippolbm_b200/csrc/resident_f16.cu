@@ -8,6 +8,6 @@ cudaError_t resident_f16(const ResidentArgs& a, int walls, cudaStream_t s) {
   return launch_resident<__half, float, false>(a, walls, s);
 }
 HLBM_OBSERVE_ENTRY(f16) {
-  return launch_observe<__half, float, false>(fin, flags, p, blocks, partials, done, out, s);
+  return launch_observe<__half, float, false>(fin, fout, flags, p, blocks, partials, done, out, s);
 }
 }  // namespace hlbm

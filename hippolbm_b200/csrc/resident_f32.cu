@@ -8,6 +8,6 @@ cudaError_t resident_f32(const ResidentArgs& a, int walls, cudaStream_t s) {
   return launch_resident<float, float, false>(a, walls, s);
 }
 HLBM_OBSERVE_ENTRY(f32) {
-  return launch_observe<float, float, false>(fin, flags, p, blocks, partials, done, out, s);
+  return launch_observe<float, float, false>(fin, fout, flags, p, blocks, partials, done, out, s);
 }
 }  // namespace hlbm

@@ -8,6 +8,6 @@ cudaError_t resident_f64(const ResidentArgs& a, int walls, cudaStream_t s) {
   return launch_resident<double, double, false>(a, walls, s);
 }
 HLBM_OBSERVE_ENTRY(f64) {
-  return launch_observe<double, double, false>(fin, flags, p, blocks, partials, done, out, s);
+  return launch_observe<double, double, false>(fin, fout, flags, p, blocks, partials, done, out, s);
 }
 }  // namespace hlbm

@@ -8,6 +8,6 @@ cudaError_t resident_f64_strict(const ResidentArgs& a, int walls, cudaStream_t s
   return launch_resident<double, double, true>(a, walls, s);
 }
 HLBM_OBSERVE_ENTRY(f64_strict) {
-  return launch_observe<double, double, true>(fin, flags, p, blocks, partials, done, out, s);
+  return launch_observe<double, double, true>(fin, fout, flags, p, blocks, partials, done, out, s);
 }
 }  // namespace hlbm
