@@ -185,13 +185,19 @@ __device__ __forceinline__ V ld_stream(const V* p) {
   else
     return *p;
 }
-// LIVE: the lattice is written by other SMs inside this launch (the resident kernel).
-template <bool LIVE, typename V>
+// How a kernel reads populations: LOAD_QUIET, a kernel that no other launch overlaps (batches, variants 6 and
+// 7): the read-only path; LOAD_WAIT, one that waits for the launch before it; LOAD_LIVE, one whose
+// own launch writes them from other SMs (the resident kernel).  Batches of ten mixed lattices by the tile-list
+// kernel (us a step, LOAD_QUIET / LOAD_WAIT): FP32 238 / 293, FP64 290 / 297.
+enum PopLoad : int { LOAD_QUIET = 0, LOAD_WAIT = 1, LOAD_LIVE = 2 };
+template <int LOAD, typename V>
 __device__ __forceinline__ V ld_pop(const V* p) {
-  if constexpr (LIVE)
+  if constexpr (LOAD == LOAD_LIVE)
     return ld_l2(p);
-  else
+  else if constexpr (LOAD == LOAD_WAIT)
     return ld_stream(p);
+  else
+    return __ldg(p);
 }
 
 // ------------------------------------------------------------------ storage rounding
@@ -821,32 +827,22 @@ __device__ __forceinline__ bool on_face(int x, int y, int z, const StepPlan& p) 
 // post_bounce_back over the non-periodic faces in launcher order x0, xl, y0, yl, z0, zl
 // (post_bounce_back.cu:115-120): the value saved by pre_bounce_back is this node's own
 // post-collision opposite population, plus the cavity increments of that face.
-template <typename S, typename R, bool LIVE>
-__device__ __forceinline__ void post_bb(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z,
-                                        const StepPlan& p) {
+// A leading post_bounce_back (`restore` false, OP_CAVITY): the pulled values are the ones it restores, so
+// only the increments are added, to the values in hand.
+template <typename S, typename R, int LOAD>
+__device__ __forceinline__ void post_bb(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z, const StepPlan& p,
+                                        bool restore) {
   Unroll<0, 6>::run([&]<int F>() {
     if (p.periodic[F / 2]) return;
     if (!on_face<F>(x, y, z, p)) return;
+    if (!restore && p.ncav[F] == 0) return;
     Unroll<0, 5>::run([&]<int K>() {
       constexpr int dst = PlaneBB::post[F][K], src = PlaneBB::pre[F][K];
-      R val = Codec<S, R>::template dec<src>(ld_pop<LIVE>(fin + src * p.stride + idx), p);
+      R val = v[dst];
+      if (restore) val = Codec<S, R>::template dec<src>(ld_pop<LOAD>(fin + src * p.stride + idx), p);
       for (int c = 0; c < p.ncav[F]; c++) val = val + R(p.cav[F][c][K]);
       v[dst] = val;
     });
-  });
-}
-
-// The cavity increments of a leading post_bounce_back (OP_CAVITY): the pulled values are the ones
-// it restores, so each increment adds to the value in hand.
-template <typename R>
-__device__ __forceinline__ void cavity_increments(R (&v)[Q], int z, const StepPlan& p) {
-  Unroll<4, 6>::run([&]<int F>() {
-    if (p.periodic[2] || z != (F == 4 ? 0 : p.nz - 1)) return;
-    for (int c = 0; c < p.ncav[F]; c++)
-      Unroll<0, 5>::run([&]<int K>() {
-        constexpr int dst = PlaneBB::post[F][K];
-        v[dst] = v[dst] + R(p.cav[F][c][K]);
-      });
   });
 }
 
@@ -895,17 +891,13 @@ __device__ __forceinline__ void zero_gradient_node(S* fin, const int8_t* __restr
   });
 }
 
-template <typename S, typename R, bool LIVE>
+template <typename S, typename R, int LOAD>
 __device__ __forceinline__ void plane_ops(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z,
                                           int8_t flag, const StepPlan& p) {
   for (int o = 0; o < p.nops; o++) {
     const PlaneOp& op = p.ops[o];
-    if (op.kind == OP_POST_BB) {
-      post_bb<S, R, LIVE>(v, fin, idx, x, y, z, p);
-      continue;
-    }
-    if (op.kind == OP_CAVITY) {
-      cavity_increments<R>(v, z, p);
+    if (op.kind == OP_POST_BB || op.kind == OP_CAVITY) {
+      post_bb<S, R, LOAD>(v, fin, idx, x, y, z, p, op.kind == OP_POST_BB);
       continue;
     }
     if (op.kind == OP_ZERO_GRADIENT) continue;  // applied by the outlet pass before the step
@@ -1047,13 +1039,13 @@ __device__ __forceinline__ bool on_op_z_face(const StepPlan& p, int z) {
 // (`pulled` false for a first step, which collides the initial state), start_iteration boxes,
 // collision.  The 16-bit tiers carry scaled deviations; the boundary operators and the boxes work
 // on full populations, so those nodes convert around them.
-template <typename S, typename R, bool STRICT, int MODE, int COLL, bool LIVE = false>
+template <typename S, typename R, bool STRICT, int MODE, int COLL, int LOAD = LOAD_WAIT>
 __device__ __forceinline__ void node_update(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z,
                                             int8_t flag, const StepPlan& p, bool pulled, bool edge) {
   constexpr bool DEV = is_16bit<S>();
   if (pulled && edge && p.nops > 0) {
     if constexpr (DEV) Unroll<0, Q>::run([&]<int I>() { v[I] = fmaf(v[I], R(p.inv_scale), R(p.dref[I])); });
-    plane_ops<S, R, LIVE>(v, fin, idx, x, y, z, flag, p);
+    plane_ops<S, R, LOAD>(v, fin, idx, x, y, z, flag, p);
     if constexpr (DEV) Unroll<0, Q>::run([&]<int I>() { v[I] = (v[I] - R(p.dref[I])) * R(p.scale); });
   }
   if (MODE != MODE_FINISH) {
@@ -1082,7 +1074,7 @@ __device__ __forceinline__ void pair_update(float2 (&v)[Q], const StepPlan& p, i
     Unroll<0, Q>::run([&]<int I>() { v[I] = Lanes<float2>::select(wall, Lanes<float2>::splat(wall_value<S, I>(p)), v[I]); });
 }
 
-template <typename S, bool WALLS, bool LIVE, bool INNER>
+template <typename S, bool WALLS, int LOAD, bool INNER>
 __device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls);
@@ -1090,24 +1082,24 @@ __device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict
 // The stored values the node (x, y, z) gathers (pull with periodic wrap and on-node bounce-back;
 // in the prologue its own values), every load issued before any is used.  A bounced value (the
 // node's own opp(I) slot) decodes like a pulled one because the storage reference is symmetric.
-template <typename S, int MODE, bool WALLS>
+template <typename S, int MODE, bool WALLS, int LOAD = LOAD_WAIT, bool INNER = true>
 __device__ __forceinline__ void node_gather(const S* fin, const int8_t* __restrict__ flags,
                                             const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q]) {
   if constexpr (MODE == MODE_PROLOGUE) {
-    Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_stream(fin + I * p.stride + idx); });
+    Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<LOAD>(fin + I * p.stride + idx); });
   } else {
-    node_pull<S, WALLS, false, true>(fin, flags, p, x, y, z, idx, raw, true);
+    node_pull<S, WALLS, LOAD, INNER>(fin, flags, p, x, y, z, idx, raw, true);
   }
 }
 
 // node_gather's pull: source coordinates x - e for e in {+1, 0, -1}; periodic axes wrap, others
 // flag "outside" (on-node bounce-back), as do wall sources where wall_bounce_back is active (WALLS
 // and, in kernels that take several plans, `walls`).  INNER: a warp of inner nodes takes a shorter way.
-template <typename S, bool WALLS, bool LIVE, bool INNER>
+template <typename S, bool WALLS, int LOAD, bool INNER>
 __device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict__ flags,
                                           const StepPlan& p, int x, int y, int z, int64_t idx, S (&raw)[Q],
                                           bool walls) {
-  if constexpr (INNER && !LIVE && sizeof(S) < 8) {
+  if constexpr (INNER && LOAD != LOAD_LIVE && sizeof(S) < 8) {
     // A warp of inner nodes needs one constant offset per direction: about 250 instructions of index
     // arithmetic less a node (the one-node FP32 step of a 181 x 150 x 170 channel is bound by issue).
     // Decided per warp: lanes that went different ways would wait for each other's loads.  Measured (us a
@@ -1117,11 +1109,11 @@ __device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict
     const bool inner = x > 0 && x < p.nx - 1 && y > 0 && y < p.ny - 1 && z > 0 && z < p.nz - 1;
     if (__all_sync(__activemask(), inner)) {
       const S* at = fin + idx;
-      Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<LIVE>(at + p.pull[I]); });
+      Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<LOAD>(at + p.pull[I]); });
       if constexpr (WALLS) {
         if (walls && (p.nearwall == nullptr || p.nearwall[idx] != 0))
           Unroll<1, Q>::run([&]<int I>() {
-            if (flags[idx + p.pull[I] - I * p.stride] == FLAG_WALL) raw[I] = ld_pop<LIVE>(at + D3Q19::opp(I) * p.stride);
+            if (flags[idx + p.pull[I] - I * p.stride] == FLAG_WALL) raw[I] = ld_pop<LOAD>(at + D3Q19::opp(I) * p.stride);
           });
       }
       return;
@@ -1147,14 +1139,19 @@ __device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict
     sy[k] = cy;
     sz[k] = cz;
   }
+  // The tile-list kernel decides every bounce before it loads: with the sources kept for a test after the
+  // loads its FP16 form spilled 396 bytes a thread (252 -> 487 us a step of ten lattices).
+  constexpr bool TEST_FIRST = WALLS && LOAD == LOAD_QUIET;
+  const bool near_first = TEST_FIRST && walls && (p.nearwall == nullptr || p.nearwall[idx] != 0);
   Unroll<0, Q>::run([&]<int I>() {
     constexpr int kx = 1 - D3Q19::ex[I], ky = 1 - D3Q19::ey[I], kz = 1 - D3Q19::ez[I];
     constexpr int O = D3Q19::opp(I);
-    const bool bounce = ox[kx] || oy[ky] || oz[kz];
+    bool bounce = ox[kx] || oy[ky] || oz[kz];
     const int64_t src = ((int64_t)sz[kz] * p.ny + sy[ky]) * p.nx + sx[kx];
-    raw[I] = ld_pop<LIVE>(bounce ? fin + O * p.stride + idx : fin + I * p.stride + src);
+    if (TEST_FIRST && I != 0 && !bounce && near_first) bounce = flags[src] == FLAG_WALL;
+    raw[I] = ld_pop<LOAD>(bounce ? fin + O * p.stride + idx : fin + I * p.stride + src);
   });
-  if constexpr (WALLS) {
+  if constexpr (WALLS && !TEST_FIRST) {
     // next to a wall: the values just pulled from wall nodes give way to the node's own (after all
     // loads are on their way, so that none waits for the map)
     if (walls && (p.nearwall == nullptr || p.nearwall[idx] != 0))
@@ -1163,20 +1160,21 @@ __device__ __forceinline__ void node_pull(const S* fin, const int8_t* __restrict
         constexpr int O = D3Q19::opp(I);
         if (ox[kx] || oy[ky] || oz[kz]) return;
         if (flags[((int64_t)sz[kz] * p.ny + sy[ky]) * p.nx + sx[kx]] == FLAG_WALL)
-          raw[I] = ld_pop<LIVE>(fin + O * p.stride + idx);
+          raw[I] = ld_pop<LOAD>(fin + O * p.stride + idx);
       });
   }
 }
 
 // The whole step for the node (x, y, z): gather, boundary operators (unless OPS is false: a face
 // pass applies them), start_iteration boxes, collision, store.
-template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL, bool OPS = true>
+template <typename S, typename R, bool STRICT, int MODE, bool WALLS, int COLL, bool OPS = true, int LOAD = LOAD_WAIT,
+          bool INNER = true>
 __device__ __forceinline__ void node_step(const S* fin, S* __restrict__ fout,
                                           const int8_t* __restrict__ flags, const StepPlan& p, int x, int y, int z) {
   const int64_t idx = ((int64_t)z * p.ny + y) * p.nx + x;
   const int8_t flag = flags[idx];
   S raw[Q];
-  node_gather<S, MODE, WALLS>(fin, flags, p, x, y, z, idx, raw);
+  node_gather<S, MODE, WALLS, LOAD, INNER>(fin, flags, p, x, y, z, idx, raw);
   if (WALLS && flag == FLAG_WALL) {
     if (MODE == MODE_FINISH)
       Unroll<0, Q>::run([&]<int I>() { fout[I * p.stride + idx] = Codec<S, R>::template enc<I>(R(0), p); });
@@ -1184,7 +1182,7 @@ __device__ __forceinline__ void node_step(const S* fin, S* __restrict__ fout,
   }
   R v[Q];
   Unroll<0, Q>::run([&]<int I>() { v[I] = load_value<S, R, I>(raw[I], p); });
-  node_update<S, R, STRICT, MODE, COLL>(v, fin, idx, x, y, z, flag, p, MODE != MODE_PROLOGUE,
+  node_update<S, R, STRICT, MODE, COLL, LOAD>(v, fin, idx, x, y, z, flag, p, MODE != MODE_PROLOGUE,
                                         OPS && on_op_face(p, x, y, z));
   store_node<S, R, MODE>(v, p, launch_seed<S>(p), idx, [&]<int I>(S s) { fout[I * p.stride + idx] = s; });
 }
@@ -1399,7 +1397,7 @@ __global__ void __launch_bounds__(FIX_THREADS)
     const int8_t flag = flags[idx];
     const bool walls = near || !g.list;
     S raw[Q];
-    node_pull<S, WALLS, false, WALLS>(fin, flags, p, x, y, z, idx, raw, walls);
+    node_pull<S, WALLS, LOAD_WAIT, WALLS>(fin, flags, p, x, y, z, idx, raw, walls);
     Unroll<0, Q>::run([&]<int I>() { v[I] = load_value<S, R, I>(raw[I], p); });
     node_update<S, R, STRICT, MODE_FUSED, COLL>(v, fin, idx, x, y, z, flag, p, true, on_op_face(p, x, y, z));
     if (WALLS && walls && flag == FLAG_WALL) live = false;

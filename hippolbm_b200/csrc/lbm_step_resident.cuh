@@ -152,7 +152,7 @@ __device__ __forceinline__ void resident_face(const S* fin, const int8_t* __rest
   }
   it.idx = (uint32_t(it.z) * uint32_t(p.ny) + uint32_t(it.y)) * uint32_t(p.nx) + uint32_t(it.x);
   it.flag = flags[it.idx];
-  node_pull<S, WALLS, true, false>(fin, flags, p, it.x, it.y, it.z, it.idx, raw, walls);
+  node_pull<S, WALLS, LOAD_LIVE, false>(fin, flags, p, it.x, it.y, it.z, it.idx, raw, walls);
 }
 
 // The update and store of a fetched node (a wall node keeps its scratch).
@@ -162,7 +162,7 @@ __device__ __forceinline__ void resident_finish(const S* fin, S* fout, const Ste
   if (WALLS && walls && it.flag == FLAG_WALL) return;
   R v[Q];
   Unroll<0, Q>::run([&]<int I>() { v[I] = load_value<S, R, I>(raw[I], p); });
-  node_update<S, R, STRICT, MODE_FUSED, 2, true>(v, fin, it.idx, it.x, it.y, it.z, it.flag, p, true, edge);
+  node_update<S, R, STRICT, MODE_FUSED, 2, LOAD_LIVE>(v, fin, it.idx, it.x, it.y, it.z, it.flag, p, true, edge);
   store_node<S, R, MODE_FUSED>(v, p, p.seed, it.idx, [&]<int I>(S s) { fout[I * p.stride + it.idx] = s; });
 }
 
@@ -202,8 +202,8 @@ __device__ __forceinline__ void resident_pair(const S* fin, S* fout, const int8_
   uint32_t w[Q];
   Unroll<0, Q>::run([&]<int I>() {
     const int e = g.off[I] + int(n);  // planes start at even elements, so parity is the offset's
-    const uint32_t w0 = ld_pop<true>(words + (e >> 1));
-    w[I] = (e & 1) ? __byte_perm(w0, ld_pop<true>(words + (e >> 1) + 1), 0x5432) : w0;
+    const uint32_t w0 = ld_pop<LOAD_LIVE>(words + (e >> 1));
+    w[I] = (e & 1) ? __byte_perm(w0, ld_pop<LOAD_LIVE>(words + (e >> 1) + 1), 0x5432) : w0;
   });
   const unsigned short fl = __ldg(reinterpret_cast<const unsigned short*>(flags + n));
   const int8_t fa = int8_t(fl & 0xff), fb = int8_t(fl >> 8);
@@ -212,11 +212,11 @@ __device__ __forceinline__ void resident_pair(const S* fin, S* fout, const int8_
       const unsigned short near = __ldg(reinterpret_cast<const unsigned short*>(p.nearwall + n));
       S raw[Q];
       if (a && (near & 0xff) == 1) {
-        node_pull<S, true, true, false>(fin, flags, p, x, y, z, n, raw, true);
+        node_pull<S, true, LOAD_LIVE, false>(fin, flags, p, x, y, z, n, raw, true);
         Unroll<0, Q>::run([&]<int I>() { w[I] = (w[I] & 0xffff0000u) | uint32_t(PackedChunk<S, 2>::bits(raw[I])); });
       }
       if (b && (near >> 8) == 1) {
-        node_pull<S, true, true, false>(fin, flags, p, x + 1, y, z, n + 1, raw, true);
+        node_pull<S, true, LOAD_LIVE, false>(fin, flags, p, x + 1, y, z, n + 1, raw, true);
         Unroll<0, Q>::run([&]<int I>() { w[I] = (w[I] & 0xffffu) | uint32_t(PackedChunk<S, 2>::bits(raw[I])) << 16; });
       }
     }
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(RES_THREADS, 1)
       const S* fin = static_cast<const S*>(L.f[cur0 ^ (k & 1)]);
       S* fout = static_cast<S*>(L.f[cur0 ^ (k & 1) ^ 1]);
       if (live) {
-        Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<true>(fin + src[I]); });
+        Unroll<0, Q>::run([&]<int I>() { raw[I] = ld_pop<LOAD_LIVE>(fin + src[I]); });
         resident_finish<S, R, STRICT, WALLS>(fin, fout, p, walls, it, raw, edge);
       }
       ok = step_done(k);

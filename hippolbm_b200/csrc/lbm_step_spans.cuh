@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1), MINB)
         live++;
         if (!face) return;
         S raw[Q];
-        node_pull<S, false, false, false>(pl.in[0], flags, p, xj, yj, zj, int64_t(n) + J, raw, false);
+        node_pull<S, false, LOAD_WAIT, false>(pl.in[0], flags, p, xj, yj, zj, int64_t(n) + J, raw, false);
         Unroll<0, Q>::run([&]<int I>() {
           const uint32_t b = uint32_t(PackedChunk<S, 2>::bits(raw[I]));
           uint32_t& w = words[I][J / 2];

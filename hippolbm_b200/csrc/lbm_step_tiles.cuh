@@ -37,9 +37,9 @@ __global__ void __launch_bounds__(256, MINB)
   for (int n = threadIdx.x; n < nodes; n += blockDim.x) {
     const int r = n / p.nx, x = n - r * p.nx;
     if (L.prologue)
-      node_step<S, R, STRICT, MODE_PROLOGUE, WALLS, 2>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
+      node_step<S, R, STRICT, MODE_PROLOGUE, WALLS, 2, true, LOAD_QUIET, false>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
     else
-      node_step<S, R, STRICT, MODE_FUSED, WALLS, 2>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
+      node_step<S, R, STRICT, MODE_FUSED, WALLS, 2, true, LOAD_QUIET, false>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
   }
 }
 
@@ -76,9 +76,9 @@ __global__ void __launch_bounds__(256, MINB)
     for (int n = threadIdx.x; n < nodes; n += blockDim.x) {
       const int r = n / p.nx, x = n - r * p.nx;
       if (L.prologue)
-        node_step<S, R, STRICT, MODE_PROLOGUE, WALLS, 2>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
+        node_step<S, R, STRICT, MODE_PROLOGUE, WALLS, 2, true, LOAD_QUIET, false>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
       else
-        node_step<S, R, STRICT, MODE_FUSED, WALLS, 2>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
+        node_step<S, R, STRICT, MODE_FUSED, WALLS, 2, true, LOAD_QUIET, false>(fin, fout, L.flags, p, x, tl.z + r, tl.y);
     }
   }
 }

@@ -293,11 +293,11 @@ __global__ void __launch_bounds__(TMA_THREADS, MINB)
           bounce = L.flags[(int64_t(sz) * ny + sy) * nx + xs] == FLAG_WALL;
         }
         if (bounce)
-          v[I] = load_value<S, R, O>(ld_stream(fin + O * stride + idx), p);
+          v[I] = load_value<S, R, O>(ld_pop<LOAD_QUIET>(fin + O * stride + idx), p);
         else
           v[I] = load_value<S, R, I>(row[xs], p);
       });
-      node_update<S, R, STRICT, MODE_FUSED, 2>(v, fin, idx, x, y, z, flag, p, !first, on_op_face(p, x, y, z));
+      node_update<S, R, STRICT, MODE_FUSED, 2, LOAD_QUIET>(v, fin, idx, x, y, z, flag, p, !first, on_op_face(p, x, y, z));
       store_node<S, R, MODE_FUSED>(v, p, p.seed, idx, [&]<int I>(S s) { fout[I * stride + idx] = s; });
     }
     __syncwarp();

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) k_observe(const S* fin, S* __restrict__ f
       const int64_t rem = idx - z * plane;
       const int y = int(rem / p.nx), x = int(rem - int64_t(y) * p.nx);
       S raw[Q];
-      node_pull<S, WALLS, false, true>(fin, flags, p, x, y, z, idx, raw, true);
+      node_pull<S, WALLS, LOAD_WAIT, true>(fin, flags, p, x, y, z, idx, raw, true);
       R v[Q];
       Unroll<0, Q>::run([&]<int I>() { v[I] = load_value<S, R, I>(raw[I], p); });
       node_update<S, R, STRICT, MODE_FINISH, 2>(v, fin, idx, x, y, z, flag, p, true, on_op_face(p, x, y, z));
