@@ -120,6 +120,9 @@ inline constexpr int variant_minb(int variant) { return variant / 2 + 1; }
 inline bool vec_eligible_bytes(const StepPlan& p, int walls, int bytes, int variant) {
   (void)walls;  // wall obstacles: the fix-up follows the vectorised kernel
   const int npt = vec_npt_bytes(bytes, variant_minb(variant));
+  // FP32 with a body force: 8-byte vectors are slower than the one-node kernel (130 x 97 x 113 MRT 100 us a step
+  // against 56, 256 x 128 x 128 BGK 176 against 140), 16-byte ones faster (134)
+  if (bytes == 4 && npt == 2 && p.has_force) return false;
   return p.nx % npt == 0 && p.nx / npt >= 32 && p.ncell <= int64_t(0xffffffffu) && pair_kernels_apply(p, bytes);
 }
 

@@ -62,3 +62,23 @@ def test_calls_of_one_step_are_quick(precision):
     for lat in lats:
         lat.close()
     assert best[0] <= 1.2 * best[1]
+
+
+@pytest.mark.parametrize("nodes,collision", [((130, 97, 113), "mrt"), ((256, 128, 128), "bgk")], ids=str)
+def test_forced_fp32_variants_are_not_slower_than_one_node(nodes, collision):
+    from hippolbm_b200.deck import poiseuille_case
+    from hippolbm_b200.lattice import Lattice
+
+    lats = [Lattice.from_case(poiseuille_case(nodes, 0.8, 1e-5, 0, collision), "f32").tune(v) for v in (4, 1, 3, 5)]
+    best = [1e9] * len(lats)
+    for _ in range(4):
+        for k, lat in enumerate(lats):
+            lat.step(2)
+            lat.sync()
+            t = time.perf_counter()
+            lat.step(60)
+            lat.sync()
+            best[k] = min(best[k], time.perf_counter() - t)
+    for lat in lats:
+        lat.close()
+    assert max(best[1:]) <= 1.15 * best[0]
