@@ -117,12 +117,14 @@ constexpr int vec_npt() {
   return vec_npt_bytes(int(sizeof(S)), MINB);
 }
 
-inline void vec_geometry(const StepPlan& p, int npt, int block_x, dim3& grid, dim3& block) {
+// Threads of the vectorised kernel in x: whole warps, as many as divide the row's and leave 256 threads a
+// block.  A row of three warps as one block of two rows (`three`) is the better form of some variants.  Measured
+// (us a step, one warp / three, couette nx x 100 x 100 BGK): FP64 variant 1 nx = 130 166 / 120, variant 3 110 /
+// 127, variant 5 180 / 175; FP32 variant 1 nx = 272 109 / 123, variant 3 nx = 130 82 / 74, variant 5 65 / 64.
+inline void vec_geometry(const StepPlan& p, int npt, bool three, dim3& grid, dim3& block) {
   const int nvec = p.nx / npt;
-  // whole warps in x, as many as divide the row's and leave 256 threads a block: 80 vectors (nx = 320 in
-  // FP32) as 3 warps of a row each would make blocks of 192 threads
   const int warps = (nvec + 31) / 32;
-  const int bx = block_x > 0 ? block_x : 32 * (warps % 4 == 0 ? 4 : (warps % 2 == 0 ? 2 : 1));
+  const int bx = 32 * (warps == 3 && three ? 3 : (warps % 4 == 0 ? 4 : (warps % 2 == 0 ? 2 : 1)));
   const int by = 256 / bx > 0 ? 256 / bx : 1;
   block = dim3(bx, by, 1);
   grid = dim3((nvec + bx - 1) / bx, (p.ny + by - 1) / by, p.nz);
@@ -133,7 +135,7 @@ cudaError_t launch_vec(int walls, const void* fin, void* fout, const int8_t* fla
                        cudaStream_t s) {
   constexpr int NPT = vec_npt<S, MINB>();
   dim3 grid, block;
-  vec_geometry(p, NPT, 0, grid, block);
+  vec_geometry(p, NPT, sizeof(S) == 8 ? MINB != 2 : sizeof(S) == 4 && MINB != 1, grid, block);
   const S* fi = static_cast<const S*>(fin);
   S* fo = static_cast<S*>(fout);
   const Planes<S> pl = make_planes(fi, fo, p.stride);
