@@ -7,7 +7,7 @@
 //   POSTCOL f[cur] holds C_{k-1}, the post-collision state inside step k (what the fused
 //           kernel carries from launch to launch);
 //   MATER   as POSTCOL, and f[1-cur] also holds S_k, produced by the finish kernel for a
-//           read-out (the next step overwrites it).
+//           read-out or by the statistics of a large lattice (the next step overwrites it).
 #include <cuda_runtime.h>
 
 #include <algorithm>

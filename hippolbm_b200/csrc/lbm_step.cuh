@@ -827,8 +827,6 @@ __device__ __forceinline__ bool on_face(int x, int y, int z, const StepPlan& p) 
 // post_bounce_back over the non-periodic faces in launcher order x0, xl, y0, yl, z0, zl
 // (post_bounce_back.cu:115-120): the value saved by pre_bounce_back is this node's own
 // post-collision opposite population, plus the cavity increments of that face.
-// A leading post_bounce_back (`restore` false, OP_CAVITY): the pulled values are the ones it restores, so
-// only the increments are added, to the values in hand.
 template <typename S, typename R, int LOAD>
 __device__ __forceinline__ void post_bb(R (&v)[Q], const S* fin, int64_t idx, int x, int y, int z, const StepPlan& p,
                                         bool restore) {
@@ -843,6 +841,20 @@ __device__ __forceinline__ void post_bb(R (&v)[Q], const S* fin, int64_t idx, in
       for (int c = 0; c < p.ncav[F]; c++) val = val + R(p.cav[F][c][K]);
       v[dst] = val;
     });
+  });
+}
+
+// The cavity increments of a leading post_bounce_back (OP_CAVITY): the pulled values are the ones
+// it restores, so each increment adds to the value in hand (post_bb without `restore` does the same).
+template <typename R>
+__device__ __forceinline__ void cavity_increments(R (&v)[Q], int z, const StepPlan& p) {
+  Unroll<4, 6>::run([&]<int F>() {
+    if (p.periodic[2] || z != (F == 4 ? 0 : p.nz - 1)) return;
+    for (int c = 0; c < p.ncav[F]; c++)
+      Unroll<0, 5>::run([&]<int K>() {
+        constexpr int dst = PlaneBB::post[F][K];
+        v[dst] = v[dst] + R(p.cav[F][c][K]);
+      });
   });
 }
 
@@ -896,9 +908,23 @@ __device__ __forceinline__ void plane_ops(R (&v)[Q], const S* fin, int64_t idx, 
                                           int8_t flag, const StepPlan& p) {
   for (int o = 0; o < p.nops; o++) {
     const PlaneOp& op = p.ops[o];
-    if (op.kind == OP_POST_BB || op.kind == OP_CAVITY) {
-      post_bb<S, R, LOAD>(v, fin, idx, x, y, z, p, op.kind == OP_POST_BB);
-      continue;
+    // The batch kernels, whose node code is the largest, take one routine for both forms of the operator
+    // (us a step of ten lattices, one routine / two: FP32 223 / 234, FP64 variant 6 491 / 538), the others
+    // one for each (resident FP16 24 x 30 x 27 3.60 / 3.40, 41^3 4.28 / 4.12).
+    if constexpr (LOAD == LOAD_QUIET) {
+      if (op.kind == OP_POST_BB || op.kind == OP_CAVITY) {
+        post_bb<S, R, LOAD>(v, fin, idx, x, y, z, p, op.kind == OP_POST_BB);
+        continue;
+      }
+    } else {
+      if (op.kind == OP_POST_BB) {
+        post_bb<S, R, LOAD>(v, fin, idx, x, y, z, p, true);
+        continue;
+      }
+      if (op.kind == OP_CAVITY) {
+        cavity_increments<R>(v, z, p);
+        continue;
+      }
     }
     if (op.kind == OP_ZERO_GRADIENT) continue;  // applied by the outlet pass before the step
     if (flag != FLAG_FLUID) continue;  // neuman / lid functors act on fluid nodes only
